@@ -82,6 +82,27 @@ def load():
     return _lib
 
 
+_HOST_ENTRIES = ("elsa_forward_workspace_bytes", "elsa_twopass_forward", "elsa_twopass_forward_strided",
+                 "elsa_backward_workspace_bytes", "elsa_twopass_backward", "elsa_twopass_backward_strided", "elsa_strerror",
+                 "elsa_last_cuda_error")
+_host_module = None
+
+
+def host():
+    """The native host path (csrc/host.cpp), bound to the loaded library; raises RuntimeError when it has not been built."""
+    global _host_module
+    if _host_module is None:
+        lib = load()
+        try:
+            from . import _host as mod
+        except ImportError as exc:
+            raise RuntimeError(f"elsa_b200/_host.so is missing or does not load ({exc}): build it with "
+                               "`python -m elsa_b200.build`") from exc
+        mod.bind({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in _HOST_ENTRIES})
+        _host_module = mod
+    return _host_module
+
+
 def check(status: int, what: str) -> None:
     if status == 0:
         return

@@ -91,6 +91,17 @@ def _check_qkv(q, k, v, who: str):
         raise ValueError("q, k, v must share one dtype")
 
 
+def _resolve_keywords(*, block_m=None, block_n=None, q_chunk_size=None, summary_dtype=None, phase1_warps=None, phase2_warps=None,
+                      phase1_stages=None, phase2_stages=None, input_precision="auto", algorithm="auto"):
+    """The operator's keywords as the native host path takes them: (summary dtype code or -1 for the input's, partition
+    width, query chunk), after the same checks."""
+    sdt, part_width, q_chunk = _resolve_common(
+        None, algorithm=algorithm, input_precision=input_precision, summary_dtype=summary_dtype, block_m=block_m, block_n=block_n,
+        q_chunk_size=q_chunk_size, phase1_warps=phase1_warps, phase2_warps=phase2_warps, phase1_stages=phase1_stages,
+        phase2_stages=phase2_stages)
+    return -1 if sdt is None else _lib.dtype_code(sdt), part_width, q_chunk
+
+
 def _resolve_common(q, *, algorithm, input_precision, summary_dtype, block_m, block_n, q_chunk_size,
                     phase1_warps, phase2_warps, phase1_stages, phase2_stages):
     if algorithm not in ("auto", "paper_scan"):
@@ -98,8 +109,8 @@ def _resolve_common(q, *, algorithm, input_precision, summary_dtype, block_m, bl
     if input_precision not in ("auto", "ieee", "tf32", "tf32x3"):
         raise ValueError("input_precision must be 'auto', 'ieee', 'tf32', or 'tf32x3'")
     if summary_dtype is None:
-        summary_dtype = q.dtype
-    if summary_dtype not in (torch.float16, torch.bfloat16, torch.float32):
+        summary_dtype = None if q is None else q.dtype
+    if summary_dtype is not None and summary_dtype not in (torch.float16, torch.bfloat16, torch.float32):
         raise ValueError("summary_dtype must be fp16, bf16, or fp32")
     for name, val in (("phase1_warps", phase1_warps), ("phase2_warps", phase2_warps)):
         if val is not None:
@@ -274,6 +285,15 @@ def twopass_attention(
     head-dim-64 kernels (q scaled by log2(e)/8 in fp16, attention_parallel_scan.py:153-154,160) where the reference
     would run them (fp16, D = 64, no bias, not causal); by default the scale is applied exactly, in fp32.
     """
+    if not reference_rounding and isinstance(q, torch.Tensor) and q.is_cuda:
+        sdt, part_width, q_chunk = _resolve_keywords(
+            block_m=block_m, block_n=block_n, q_chunk_size=q_chunk_size, summary_dtype=summary_dtype, phase1_warps=phase1_warps,
+            phase2_warps=phase2_warps, phase1_stages=phase1_stages, phase2_stages=phase2_stages, input_precision=input_precision,
+            algorithm=algorithm)
+        out = _lib.host().attention(q, k, v, bias, is_causal, sdt, part_width, q_chunk, False)
+        if out is not None:
+            return out
+    # the general path: what the native one does not cover, and the errors
     _check_qkv(q, k, v, "twopass_attention")
     if algorithm not in ("auto", "paper_scan"):
         raise ValueError("only algorithm='paper_scan' is available in this strict release")

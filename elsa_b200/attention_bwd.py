@@ -16,7 +16,7 @@ import torch
 
 from . import _lib
 from .attention import (_DeviceScope, _aligned, _bhnd_strides, _cached_bytes, _canonical_bias, _check_qkv, _empty_like_layout, _forward_impl, _i64x,
-                        _in_place_or_copy, _resolve_common, _validate_warps)
+                        _in_place_or_copy, _resolve_common, _resolve_keywords, _validate_warps)
 
 
 def twopass_attention_with_state(
@@ -194,6 +194,15 @@ def twopass_attention_backward(
     dq, dk, dv, _ = _backward_impl(q, k, v, out.to(q.dtype), grad_out, bias=bias, is_causal=is_causal, row_m=row_m,
                                    row_z=row_z, want_dbias=False)
     return dq, dk, dv
+
+
+def _native_keywords(fwd_kwargs: dict):
+    """(summary dtype code, partition width, query chunk) for the native host path."""
+    if not fwd_kwargs:
+        return -1, 0, 0
+    if "reference_rounding" in fwd_kwargs:
+        fwd_kwargs = {name: val for name, val in fwd_kwargs.items() if name != "reference_rounding"}
+    return _resolve_keywords(**fwd_kwargs)
 
 
 class _TwopassAttentionAutograd(torch.autograd.Function):
@@ -419,7 +428,13 @@ def twopass_attention_qkvpacked(qkv: torch.Tensor, *, bias: Optional[torch.Tenso
         raise ValueError("input_precision must be 'auto', 'ieee', 'tf32', or 'tf32x3'")
     if fwd_kwargs.get("bwd_num_warps") is not None:
         _validate_warps("num_warps", fwd_kwargs["bwd_num_warps"])
-    fwd_kwargs = {name: val for name, val in fwd_kwargs.items() if not name.startswith("bwd_")}
+    if fwd_kwargs:
+        fwd_kwargs = {name: val for name, val in fwd_kwargs.items() if not name.startswith("bwd_")}
+    if qkv.is_cuda and not fwd_kwargs.get("reference_rounding", False):
+        out = _lib.host().attention_packed(qkv, bias, is_causal, *_native_keywords(fwd_kwargs), bool(train))
+        if out is not None:
+            return out
+    # the general path: what the native one does not cover, and the errors
     if not train:
         if not fwd_kwargs.get("reference_rounding", False) and _packed_fast_ok(qkv):
             bias32 = None
@@ -453,6 +468,11 @@ def twopass_attention_train(
         raise ValueError("input_precision must be 'auto', 'ieee', 'tf32', or 'tf32x3'")
     if bwd_num_warps is not None:
         _validate_warps("num_warps", bwd_num_warps)
+    if isinstance(q, torch.Tensor) and q.is_cuda and not fwd_kwargs.get("reference_rounding", False):
+        out = _lib.host().attention(q, k, v, bias, is_causal, *_native_keywords(fwd_kwargs), True)
+        if out is not None:
+            return out
+    # the general path: what the native one does not cover, and the errors
     bwd_kwargs = {name: val for name, val in (("block_m", bwd_block_m), ("block_n", bwd_block_n),
                                               ("num_warps", bwd_num_warps), ("num_stages", bwd_num_stages))
                   if val is not None}

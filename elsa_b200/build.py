@@ -1,4 +1,5 @@
-"""Ahead-of-time build of libelsa_b200.so (plain nvcc, sm_100a only, no torch headers).
+"""Ahead-of-time build of libelsa_b200.so (plain nvcc, sm_100a only, no torch headers) and of _host.so, the native host
+path of the Python operators (g++ against the headers of the installed torch).
 
     python -m elsa_b200.build            # build if sources are newer than the library
     python -m elsa_b200.build --force
@@ -14,6 +15,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(CSRC, "build")
 LIB_PATH = os.path.join(HERE, "libelsa_b200.so")
+HOST_SRC = os.path.join(CSRC, "host.cpp")
+HOST_PATH = os.path.join(HERE, "_host.so")
 SOURCES = ["api.cu", "phase2.cu", "fold_simt.cu", "bwd_simt.cu", "fold_tc.cu", "fold_tc3.cu", "fold_tcw.cu", "bwd_tc.cu", "bwd_tc3.cu", "bwd_tcw.cu", "win_tc.cu", "peaks.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -38,7 +41,32 @@ def needs_build() -> bool:
     return not os.path.exists(LIB_PATH) or os.path.getmtime(LIB_PATH) < _newest_source_mtime()
 
 
+def host_needs_build() -> bool:
+    newest = max(os.path.getmtime(HOST_SRC), os.path.getmtime(os.path.join(os.path.dirname(HERE), "include", "elsa_b200.h")))
+    return not os.path.exists(HOST_PATH) or os.path.getmtime(HOST_PATH) < newest
+
+
+def build_host() -> None:
+    import sysconfig
+
+    import torch
+    root = torch.__path__[0]
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    lib = os.path.join(root, "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{path}" for path in include), HOST_SRC,
+           "-o", HOST_PATH, f"-L{lib}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10",
+           f"-Wl,-rpath,{lib}"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for host.cpp:\n{res.stdout}\n{res.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    if force or host_needs_build():
+        build_host()
     if not force and not needs_build():
         return LIB_PATH
     os.makedirs(OBJ_DIR, exist_ok=True)
