@@ -97,6 +97,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   __shared__ int abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.y;
   const int bi = bh / prm.heads, hi = bh - bi * prm.heads;   // tensor-map coordinates of this (batch*head)
   const int k0 = blockIdx.x * 128;                  // first (local) key row of this CTA
@@ -154,7 +155,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
   auto tS = [&](int h) { return tmem_base + 64 * h; };
   auto tdP = [&](int h) { return tmem_base + 128 + 64 * h; };
 
-  if (warp >= 12) {
+  if (warp_u >= 12) {
     reg_dec<80>();
     if (warp == 12 && lane == 0) {
       // ---------------- TMA producer ----------------
@@ -179,7 +180,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           tma_prefetch_l2_4d(&tmap_do, 0, qrow + kPrefetchAhead * 128, hi, bi);
         }
       }
-    } else if (warp == 13 && lane == 0) {
+    } else if (warp_u == 13) {
+      const bool leader = elect_one();
       // ---------------- MMA issuer ----------------
       constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
       constexpr uint32_t idesc_kv = make_idesc(fmt, 0, 1, 128, 64);   // dV, dK: A in TMEM, B MN-major
@@ -212,18 +214,18 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       auto issue_dkv = [&](auto ST, auto H, uint32_t acc) {
         constexpr int st = decltype(ST)::value, h = decltype(H)::value;
         // K-steps of 16 queries: P^T at columns 0, 8 (chunk 0) and 32, 40 (chunk 1); dS^T 16 columns further
-        mma_ts_x4_cols<8, 32, 40, 128>(tdV, tdP(h), ddo_mn[st][h], idesc_kv, acc);
-        mma_ts_x4_cols<8, 32, 40, 128>(tdK, tdP(h) + 16, dq_mn[st][h], idesc_kv, acc);
+        if (leader) mma_ts_x4_cols<8, 32, 40, 128>(tdV, tdP(h), ddo_mn[st][h], idesc_kv, acc);
+        if (leader) mma_ts_x4_cols<8, 32, 40, 128>(tdK, tdP(h) + 16, dq_mn[st][h], idesc_kv, acc);
       };
-      bool ok = mbar_wait(bar_kv, 0, &abort_flag, prm.status, BAR_KV) &&
-                mbar_wait(bar_kvt, 0, &abort_flag, prm.status, BAR_KVT) &&
-                (n_it == 0 || mbar_wait(bar_q_full(0), 0, &abort_flag, prm.status, BAR_Q_FULL));
+      bool ok = mbar_wait_warp(bar_kv, 0, &abort_flag, prm.status, BAR_KV) &&
+                mbar_wait_warp(bar_kvt, 0, &abort_flag, prm.status, BAR_KVT) &&
+                (n_it == 0 || mbar_wait_warp(bar_q_full(0), 0, &abort_flag, prm.status, BAR_Q_FULL));
       if (ok && n_it > 0) {
         tc_fence_after();
-        mma_ts_x4<8, 2>(tS0, tK, dq_k[0], idesc_st, 0u);
-        mma_commit(bar_s);
-        mma_ts_x4<8, 2>(tdP0, tV, ddo_k[0], idesc_st, 0u);
-        mma_commit(bar_dpx(0));
+        if (leader) mma_ts_x4<8, 2>(tS0, tK, dq_k[0], idesc_st, 0u);
+        if (leader) mma_commit(bar_s);
+        if (leader) mma_ts_x4<8, 2>(tdP0, tV, ddo_k[0], idesc_st, 0u);
+        if (leader) mma_commit(bar_dpx(0));
       }
       // One iteration on ring stage ST (the next one is on the other stage).  S^T of the NEXT query tile is issued
       // as soon as the compute warps hold the current S^T in registers (their exp2 phase then overlaps the
@@ -232,24 +234,24 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       // dV / dK / dP^T stand between the halves' arrival and the next dS phase: measured 1.95 ms against 1.59 ms.)
       auto issue_dq = [&](int it_q, auto STQ) {       // dQ of tile it_q, whose dS^T sits in buffer STQ
         constexpr int stq = decltype(STQ)::value;
-        if (it_q > 0 && !(ok = mbar_wait(bar_dq_free, (it_q - 1) & 1, &abort_flag, prm.status, BAR_DQ_FREE))) return;
-        mma_ss_x4<128, 128>(tdQ, dds[stq], bk_mn, idesc_dq, 0u);
-        mma_ss_x4<128, 128>(tdQ, dds[stq] + 512, bk_mn + 512, idesc_dq, 1u);
-        mma_commit(bar_q_free(stq));   // dQ(it_q) is complete: the drain warps may read it
+        if (it_q > 0 && !(ok = mbar_wait_warp(bar_dq_free, (it_q - 1) & 1, &abort_flag, prm.status, BAR_DQ_FREE))) return;
+        if (leader) mma_ss_x4<128, 128>(tdQ, dds[stq], bk_mn, idesc_dq, 0u);
+        if (leader) mma_ss_x4<128, 128>(tdQ, dds[stq] + 512, bk_mn + 512, idesc_dq, 1u);
+        if (leader) mma_commit(bar_q_free(stq));   // dQ(it_q) is complete: the drain warps may read it
       };
       auto iteration = [&](int it, auto ST) {
         constexpr int st = decltype(ST)::value;
         const bool more = it + 1 < n_it;
         const uint32_t pit = it & 1;
         if (more) {
-          ok = mbar_wait(bar_q_full(st ^ 1), ((it + 1) / kQStages) & 1, &abort_flag, prm.status, BAR_Q_FULL) &&
-               mbar_wait(bar_lds, pit, &abort_flag, prm.status, BAR_LDS);
+          ok = mbar_wait_warp(bar_q_full(st ^ 1), ((it + 1) / kQStages) & 1, &abort_flag, prm.status, BAR_Q_FULL) &&
+               mbar_wait_warp(bar_lds, pit, &abort_flag, prm.status, BAR_LDS);
           if (!ok) return;
           tc_fence_after();
-          mma_ts_x4<8, 2>(tS0, tK, dq_k[st ^ 1], idesc_st, 0u);
-          mma_commit(bar_s);
+          if (leader) mma_ts_x4<8, 2>(tS0, tK, dq_k[st ^ 1], idesc_st, 0u);
+          if (leader) mma_commit(bar_s);
         }
-        if (!(ok = mbar_wait(bar_pds, pit, &abort_flag, prm.status, BAR_PDS))) return;
+        if (!(ok = mbar_wait_warp(bar_pds, pit, &abort_flag, prm.status, BAR_PDS))) return;
         tc_fence_after();
         issue_dkv(ST, I0{}, it == 0 ? 0u : 1u);
         issue_dkv(ST, I1{}, 1u);
@@ -257,8 +259,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           // one commit for two facts: dP^T of the next tile is in TMEM, and dV / dK of this tile have retired, so
           // Q, dO and the row statistics of this tile are not read again (dQ takes dS^T and K) and the producer may
           // refill the ring stage
-          mma_ts_x4<8, 2>(tdP0, tV, ddo_k[st ^ 1], idesc_st, 0u);
-          mma_commit(bar_dpx(st ^ 1));
+          if (leader) mma_ts_x4<8, 2>(tdP0, tV, ddo_k[st ^ 1], idesc_st, 0u);
+          if (leader) mma_commit(bar_dpx(st ^ 1));
         }
         issue_dq(it, ST);
       };
@@ -266,7 +268,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         iteration(it, I0{});
         if (ok && it + 1 < n_it) iteration(it + 1, I1{});
       }
-      if (ok) mma_commit(bar_done);
+      if (ok && leader) mma_commit(bar_done);
     }
   } else if (warp >= 8) {
     // ---------------- dQ drain warps: one thread per query row ----------------
@@ -274,7 +276,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     for (int it = 0; it < n_it; ++it) {
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_q_free(it % kQStages), (it / kQStages) & 1, &abort_flag, prm.status, BAR_DQ_FULL))) break;
+      if (!mbar_wait_warp(bar_q_free(it % kQStages), (it / kQStages) & 1, &abort_flag, prm.status, BAR_DQ_FULL)) break;
       tc_fence_after();
       uint32_t r0[32], r1[32];
       tmem_ld32(tdQ + lane_off, r0);
@@ -320,7 +322,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
 
     // one-time copy of this CTA's K (warps 0-3) / V (warps 4-7) tile from shared memory into TMEM as the A operand
     // of S^T / dP^T: lane = key row, 32 columns of 16-bit pairs; the smem row is un-swizzled on the way
-    if (!__all_sync(0xffffffffu, mbar_wait(bar_kv, 0, &abort_flag, prm.status, BAR_KV))) alive = false;
+    if (!mbar_wait_warp(bar_kv, 0, &abort_flag, prm.status, BAR_KV)) alive = false;
     if (alive) {
       const uint8_t* src = smem_gen + ((half == 0 ? sK : sV) - smem_base) + row * 128;
       uint32_t w[32];
@@ -338,10 +340,10 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     for (int it = 0; alive && it < n_it; ++it) {
       const int st = it % kQStages;
       const int q_tile0 = (it_begin + it) * 128;
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_s, it & 1, &abort_flag, prm.status, BAR_SP))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_s, it & 1, &abort_flag, prm.status, BAR_SP)) { alive = false; break; }
       // the row statistics of this stage were written by the bulk copies that complete on q_full: observe that
       // barrier directly (it completed before the MMAs behind bar_s were issued, so this never spins)
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_q_full(st), (it / kQStages) & 1, &abort_flag, prm.status, BAR_Q_FULL))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_q_full(st), (it / kQStages) & 1, &abort_flag, prm.status, BAR_Q_FULL)) { alive = false; break; }
       tc_fence_after();
       const float4* nl4 =reinterpret_cast<const float4*>(smem_gen + (sNL(st) - smem_base)) + half * 16;
       const float4* nd4 = reinterpret_cast<const float4*>(smem_gen + (sND(st) - smem_base)) + half * 16;
@@ -377,7 +379,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       }
 
       // ---- phase B: dS^T = P^T * (dP^T - D); P^T and dS^T (16-bit) handed to dV / dK in two 32-query chunks ----
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_dpx(it & 1), (it / 2) & 1, &abort_flag, prm.status, BAR_DP))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_dpx(it & 1), (it / 2) & 1, &abort_flag, prm.status, BAR_DP)) { alive = false; break; }
       tc_fence_after();
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) {
@@ -418,7 +420,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     }
 
     // ---- epilogue: dK, dV of this key tile (tcgen05.ld is warp-collective: only the stores are predicated) ----
-    if (alive && n_it > 0 && !__all_sync(0xffffffffu, mbar_wait(bar_done, 0, &abort_flag, prm.status, BAR_DONE))) alive = false;
+    if (alive && n_it > 0 && !mbar_wait_warp(bar_done, 0, &abort_flag, prm.status, BAR_DONE)) alive = false;
     if (alive) {
       uint32_t rk[32], rv[32];
       if (n_it > 0) {

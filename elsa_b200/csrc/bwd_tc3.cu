@@ -136,6 +136,7 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   __shared__ float row_max[2][4][128];   // [tile parity][column quarter][row]: the quarter-row maxima of |dS|
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.y;
   const int q0 = blockIdx.x * 128;
   const int N = prm.n_ctx, NK = prm.n_keys, koff = prm.key_offset;
@@ -208,8 +209,9 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         }
       }
     }
-  } else if (warp == kIssuerWarp) {
-    if (n_t > 0 && lane == 0) {
+  } else if (warp_u == kIssuerWarp) {
+    if (n_t > 0) {
+      const bool leader = elect_one();
       // ---------------- MMA issuer ----------------
       constexpr uint32_t idesc_k = make_idesc(kPlaneFmt, 0, 0, 128, 128);   // S, dP: A, B K-major, N = 128 keys
       constexpr uint32_t idesc_mn = make_idesc(kPlaneFmt, 0, 1, 128, 64);   // dQ_j: A in TMEM, B (K) MN-major, N = 64 = d
@@ -218,30 +220,30 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       const uint64_t dk_k0 = make_sdesc(sKs(0), 16, 1024), dk_mn0 = make_sdesc(sKs(0), 128 * 128, 1024);
       const uint64_t dv_k0 = make_sdesc(sVs(0), 16, 1024);
       constexpr uint64_t kPlaneStep = kPlaneBytes >> 4;
-      bool ok = mbar_wait(bar_stage, 0, &abort_flag, prm.status, BAR_STAGE);
+      bool ok = mbar_wait_warp(bar_stage, 0, &abort_flag, prm.status, BAR_STAGE);
       auto issue_sdp = [&](int j) {
         bool first = true;
         for (int vp = kPlanes - 1; vp >= 0 && ok; --vp) {  // dP = dO V^T
           const int seq = kPlanes * j + kPlanes - 1 - vp, slot = seq % kDqVSlots;
-          if (!(ok = mbar_wait(bar_vfull(slot), (seq / kDqVSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
+          if (!(ok = mbar_wait_warp(bar_vfull(slot), (seq / kDqVSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
           for (int gp = kPlanes - 1 - vp; gp >= 0; --gp) {
-            mma_ss_x4<2, 2>(tdP, dDOp[gp], dv_k0 + slot * kPlaneStep, idesc_k, first ? 0u : 1u);
+            if (leader) mma_ss_x4<2, 2>(tdP, dDOp[gp], dv_k0 + slot * kPlaneStep, idesc_k, first ? 0u : 1u);
             first = false;
           }
-          mma_commit(bar_vfree(slot));
+          if (leader) mma_commit(bar_vfree(slot));
         }
         first = true;
         for (int kp = kPlanes - 1; kp >= 0 && ok; --kp) {  // S = Q K^T
           const int seq = kPlanes * j + kPlanes - 1 - kp, slot = seq % kDqKSlots;
-          if (!(ok = mbar_wait(bar_kfull(slot), (seq / kDqKSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
+          if (!(ok = mbar_wait_warp(bar_kfull(slot), (seq / kDqKSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
           for (int qp = kPlanes - 1 - kp; qp >= 0; --qp) {
-            mma_ss_x4<2, 2>(tS, dQp[qp], dk_k0 + slot * kPlaneStep, idesc_k, first ? 0u : 1u);
+            if (leader) mma_ss_x4<2, 2>(tS, dQp[qp], dk_k0 + slot * kPlaneStep, idesc_k, first ? 0u : 1u);
             first = false;
           }                                   // the K planes stay: dQ_j reads them again
         }
-        if (ok) mma_commit(bar_sdp);
+        if (ok && leader) mma_commit(bar_sdp);
       };
       if (ok) {
         tc_fence_after();
@@ -249,24 +251,24 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       }
       for (int j = 0; ok && j < n_t; ++j) {
         if (j + 1 < n_t) {
-          if (!(ok = mbar_wait(bar_sfree, j & 1, &abort_flag, prm.status, BAR_SFREE))) break;
+          if (!(ok = mbar_wait_warp(bar_sfree, j & 1, &abort_flag, prm.status, BAR_SFREE))) break;
           tc_fence_after();
           issue_sdp(j + 1);
           if (!ok) break;
         }
-        if (!(ok = mbar_wait(bar_ds, j & 1, &abort_flag, prm.status, BAR_DS))) break;
+        if (!(ok = mbar_wait_warp(bar_ds, j & 1, &abort_flag, prm.status, BAR_DS))) break;
         tc_fence_after();
         bool first = true;
         for (int kp = kPlanes - 1; kp >= 0; --kp) {        // dQ_j = dS K over the 128 keys (eight K-steps)
           const int slot = (kPlanes * j + kPlanes - 1 - kp) % kDqKSlots;
           for (int sp = kPlanes - 1 - kp; sp >= 0; --sp) {
-            mma_ts_x4<8, 128>(tdQ, tDS + 64 * sp, dk_mn0 + slot * kPlaneStep, idesc_mn, first ? 0u : 1u);
-            mma_ts_x4<8, 128>(tdQ, tDS + 64 * sp + 32, dk_mn0 + slot * kPlaneStep + 512, idesc_mn, 1u);
+            if (leader) mma_ts_x4<8, 128>(tdQ, tDS + 64 * sp, dk_mn0 + slot * kPlaneStep, idesc_mn, first ? 0u : 1u);
+            if (leader) mma_ts_x4<8, 128>(tdQ, tDS + 64 * sp + 32, dk_mn0 + slot * kPlaneStep + 512, idesc_mn, 1u);
             first = false;
           }
-          mma_commit(bar_kfree(slot));
+          if (leader) mma_commit(bar_kfree(slot));
         }
-        mma_commit(bar_dq);                   // dQ_j is complete; the dS planes may be overwritten
+        if (leader) mma_commit(bar_dq);                   // dQ_j is complete; the dS planes may be overwritten
       }
     }
   } else {
@@ -305,7 +307,7 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     };
 
     for (int j = 0; alive && j < n_t; ++j) {
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_sdp, j & 1, &abort_flag, prm.status, BAR_SDP))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_sdp, j & 1, &abort_flag, prm.status, BAR_SDP)) { alive = false; break; }
       tc_fence_after();
       float ds[32];
       {
@@ -371,7 +373,7 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         // the row's scale for this tile: the largest |dS| over its 128 keys, exchanged between the row's four threads
         row_max[j & 1][cq][row] = fmaxf(abs_max16(ds), abs_max16(ds + 16));
         mbar_arrive_warp(bar_row(qd), lane);
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_row(qd), j & 1, &abort_flag, prm.status, BAR_ROW))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_row(qd), j & 1, &abort_flag, prm.status, BAR_ROW)) { alive = false; break; }
         const float mx = fmaxf(fmaxf(row_max[j & 1][0][row], row_max[j & 1][1][row]), fmaxf(row_max[j & 1][2][row], row_max[j & 1][3][row]));
         r_scale = plane_scale(__float_as_uint(mx));
 #pragma unroll
@@ -379,7 +381,7 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       }
       if (j > 0) {
         // dQ of the previous key tile has retired: it goes into the running sum, and the dS planes are free
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_dq, (j - 1) & 1, &abort_flag, prm.status, BAR_ACC))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_dq, (j - 1) & 1, &abort_flag, prm.status, BAR_ACC)) { alive = false; break; }
         tc_fence_after();
         take_dq();
       }
@@ -392,7 +394,7 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       mbar_arrive_warp(bar_ds, lane);
     }
     if (alive && n_t > 0) {
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_dq, (n_t - 1) & 1, &abort_flag, prm.status, BAR_ACC))) alive = false;
+      if (!mbar_wait_warp(bar_dq, (n_t - 1) & 1, &abort_flag, prm.status, BAR_ACC)) alive = false;
       if (alive) {
         tc_fence_after();
         take_dq();
@@ -425,6 +427,7 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __shared__ float row_max[2][4][128];   // [tile parity][column quarter][key row]: the quarter-row maxima of |dS^T|
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.y;
   const int k0 = blockIdx.x * 128;                  // first (local) key row of this CTA
   const int N = prm.n_ctx, NK = prm.n_keys;
@@ -499,8 +502,9 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
       }
     }
-  } else if (warp == kIssuerWarp) {
-    if (n_it > 0 && lane == 0) {
+  } else if (warp_u == kIssuerWarp) {
+    if (n_it > 0) {
+      const bool leader = elect_one();
       // ---------------- MMA issuer ----------------
       constexpr uint32_t idesc_k = make_idesc(kPlaneFmt, 0, 0, 128, 64);    // S^T, dP^T: A, B K-major, N = 64 queries
       constexpr uint32_t idesc_mn = make_idesc(kPlaneFmt, 0, 1, 128, 64);   // dV_i, dK_i: A in TMEM, B MN-major, N = 64 = d
@@ -508,29 +512,29 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       for (int p = 0; p < kPlanes; ++p) { dKp[p] = make_sdesc(sK(p), 16, 1024); dVp[p] = make_sdesc(sV(p), 16, 1024); }
       constexpr int kT = 2 * kPlanes;   // ring entries per query tile
       const uint64_t dk_slot0 = make_sdesc(sSlot(0), 16, 1024), dmn_slot0 = make_sdesc(sSlot(0), 64 * 128, 1024);
-      bool ok = mbar_wait(bar_kv, 0, &abort_flag, prm.status, BAR_STAGE);
+      bool ok = mbar_wait_warp(bar_kv, 0, &abort_flag, prm.status, BAR_STAGE);
       auto issue_sdp = [&](int it) {
         bool first = true;
         for (int gp = kPlanes - 1; gp >= 0 && ok; --gp) {  // dP^T = V dO^T
           const int seq = kT * it + kPlanes - 1 - gp, slot = seq % kKvSlots;
-          if (!(ok = mbar_wait(bar_full(slot), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
+          if (!(ok = mbar_wait_warp(bar_full(slot), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
           for (int vp = kPlanes - 1 - gp; vp >= 0; --vp) {
-            mma_ss_x4<2, 2>(tdP, dVp[vp], dk_slot0 + slot * kSlotStep, idesc_k, first ? 0u : 1u);
+            if (leader) mma_ss_x4<2, 2>(tdP, dVp[vp], dk_slot0 + slot * kSlotStep, idesc_k, first ? 0u : 1u);
             first = false;
           }
         }
         first = true;
         for (int qp = kPlanes - 1; qp >= 0 && ok; --qp) {  // S^T = K Q^T
           const int seq = kT * it + kT - 1 - qp, slot = seq % kKvSlots;
-          if (!(ok = mbar_wait(bar_full(slot), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
+          if (!(ok = mbar_wait_warp(bar_full(slot), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
           for (int kp = kPlanes - 1 - qp; kp >= 0; --kp) {
-            mma_ss_x4<2, 2>(tS, dKp[kp], dk_slot0 + slot * kSlotStep, idesc_k, first ? 0u : 1u);
+            if (leader) mma_ss_x4<2, 2>(tS, dKp[kp], dk_slot0 + slot * kSlotStep, idesc_k, first ? 0u : 1u);
             first = false;
           }
         }
-        if (ok) mma_commit(bar_sdp);
+        if (ok && leader) mma_commit(bar_sdp);
       };
       if (ok) {
         tc_fence_after();
@@ -538,32 +542,32 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       for (int it = 0; ok && it < n_it; ++it) {
         if (it + 1 < n_it) {
-          if (!(ok = mbar_wait(bar_sfree, it & 1, &abort_flag, prm.status, BAR_SFREE))) break;
+          if (!(ok = mbar_wait_warp(bar_sfree, it & 1, &abort_flag, prm.status, BAR_SFREE))) break;
           tc_fence_after();
           issue_sdp(it + 1);
           if (!ok) break;
         }
-        if (!(ok = mbar_wait(bar_pl, it & 1, &abort_flag, prm.status, BAR_DS))) break;
+        if (!(ok = mbar_wait_warp(bar_pl, it & 1, &abort_flag, prm.status, BAR_DS))) break;
         tc_fence_after();
         bool first = true;
         for (int gp = kPlanes - 1; gp >= 0; --gp) {        // dV_i = P^T dO
           const int slot = (kT * it + kPlanes - 1 - gp) % kKvSlots;
           for (int pp = kPlanes - 1 - gp; pp >= 0; --pp) {
-            mma_ts_x4<8, 128>(tdV, tP + 32 * pp, dmn_slot0 + slot * kSlotStep, idesc_mn, first ? 0u : 1u);
+            if (leader) mma_ts_x4<8, 128>(tdV, tP + 32 * pp, dmn_slot0 + slot * kSlotStep, idesc_mn, first ? 0u : 1u);
             first = false;
           }
-          mma_commit(bar_free(slot));
+          if (leader) mma_commit(bar_free(slot));
         }
         first = true;
         for (int qp = kPlanes - 1; qp >= 0; --qp) {        // dK_i = dS^T Q
           const int slot = (kT * it + kT - 1 - qp) % kKvSlots;
           for (int sp = kPlanes - 1 - qp; sp >= 0; --sp) {
-            mma_ts_x4<8, 128>(tdK, tDS + 32 * sp, dmn_slot0 + slot * kSlotStep, idesc_mn, first ? 0u : 1u);
+            if (leader) mma_ts_x4<8, 128>(tdK, tDS + 32 * sp, dmn_slot0 + slot * kSlotStep, idesc_mn, first ? 0u : 1u);
             first = false;
           }
-          mma_commit(bar_free(slot));
+          if (leader) mma_commit(bar_free(slot));
         }
-        mma_commit(bar_acc);                  // dV_i, dK_i are complete; the planes may be overwritten
+        if (leader) mma_commit(bar_acc);                  // dV_i, dK_i are complete; the planes may be overwritten
       }
     }
   } else {
@@ -609,12 +613,12 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
     for (int it = 0; it < n_it; ++it) {
       const int q_tile0 = (it_begin + it) * 64;
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_sdp, it & 1, &abort_flag, prm.status, BAR_SDP))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_sdp, it & 1, &abort_flag, prm.status, BAR_SDP)) { alive = false; break; }
       // the tile's row statistics were written by the bulk copies that complete on its first slot's barrier: observe
       // that barrier directly (it completed before the MMAs behind bar_sdp were issued, so this never spins)
       {
         const int seq = 2 * kPlanes * it;
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_full(seq % kKvSlots), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_full(seq % kKvSlots), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL)) { alive = false; break; }
       }
       tc_fence_after();
       float p[16], ds[16];
@@ -661,7 +665,7 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         // the key row's scale for this tile: the largest |dS^T| over its 64 queries, exchanged between its four threads
         row_max[it & 1][cq][row] = abs_max16(ds);
         mbar_arrive_warp(bar_row(qd), lane);
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_row(qd), it & 1, &abort_flag, prm.status, BAR_ROW))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_row(qd), it & 1, &abort_flag, prm.status, BAR_ROW)) { alive = false; break; }
         const float mx = fmaxf(fmaxf(row_max[it & 1][0][row], row_max[it & 1][1][row]), fmaxf(row_max[it & 1][2][row], row_max[it & 1][3][row]));
         r_scale = plane_scale(__float_as_uint(mx));
 #pragma unroll
@@ -669,7 +673,7 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       if (it > 0) {
         // dV, dK of the previous query tile have retired: they go into the running sums, and the planes are free
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_acc, (it - 1) & 1, &abort_flag, prm.status, BAR_ACC))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_acc, (it - 1) & 1, &abort_flag, prm.status, BAR_ACC)) { alive = false; break; }
         tc_fence_after();
         take_acc();
       }
@@ -681,7 +685,7 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       mbar_arrive_warp(bar_pl, lane);
     }
     if (alive && n_it > 0) {
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_acc, (n_it - 1) & 1, &abort_flag, prm.status, BAR_ACC))) alive = false;
+      if (!mbar_wait_warp(bar_acc, (n_it - 1) & 1, &abort_flag, prm.status, BAR_ACC)) alive = false;
       if (alive) {
         tc_fence_after();
         take_acc();

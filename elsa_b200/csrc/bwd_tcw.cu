@@ -107,6 +107,7 @@ bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   __shared__ int abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.y;
   const int bi = bh / prm.heads, hi = bh - bi * prm.heads;   // tensor-map coordinates of this (batch*head)
   const int q0 = blockIdx.x * 128;
@@ -179,8 +180,9 @@ bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         }
       }
     }
-  } else if (warp == kIssuerWarp) {
-    if (n_t > 0 && lane == 0) {
+  } else if (warp_u == kIssuerWarp) {
+    if (n_t > 0) {
+      const bool leader = elect_one();
       // ---------------- MMA issuer ----------------
       constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
       constexpr uint32_t idesc_k = make_idesc(fmt, 0, 0, 128, 128);   // S, dP: A, B K-major, N = 128 keys
@@ -190,22 +192,22 @@ bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       const uint64_t dk_k0 = make_sdesc(sKs(0), 16, 1024), dk_mn0 = make_sdesc(sKs(0), 128 * 128, 1024);
       const uint64_t dv_k0 = make_sdesc(sVs(0), 16, 1024);
       const int nh = BIAS ? prm.n_halves : 2;
-      bool ok = mbar_wait(bar_stage, 0, &abort_flag, prm.status, BAR_STAGE);
+      bool ok = mbar_wait_warp(bar_stage, 0, &abort_flag, prm.status, BAR_STAGE);
       auto issue_sdp = [&](int j) {
         for (int h = 0; h < nh && ok; ++h) {               // dP = sum over the halves of dO_h V_h^T
           const int seq = 2 * j + h, slot = seq % kDqVSlots;
-          if (!(ok = mbar_wait(bar_vfull(slot), (seq / kDqVSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
+          if (!(ok = mbar_wait_warp(bar_vfull(slot), (seq / kDqVSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
-          mma_ss_x4<2, 2>(tdP, dDOh[h], dv_k0 + slot * kTileStep, idesc_k, h == 0 ? 0u : 1u);
-          mma_commit(bar_vfree(slot));
+          if (leader) mma_ss_x4<2, 2>(tdP, dDOh[h], dv_k0 + slot * kTileStep, idesc_k, h == 0 ? 0u : 1u);
+          if (leader) mma_commit(bar_vfree(slot));
         }
         for (int h = 0; h < nh && ok; ++h) {               // S = sum over the halves of Q_h K_h^T
           const int seq = 2 * j + h, slot = seq % kDqKSlots;
-          if (!(ok = mbar_wait(bar_kfull(slot), (seq / kDqKSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
+          if (!(ok = mbar_wait_warp(bar_kfull(slot), (seq / kDqKSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
-          mma_ss_x4<2, 2>(tS, dQh[h], dk_k0 + slot * kTileStep, idesc_k, h == 0 ? 0u : 1u);
+          if (leader) mma_ss_x4<2, 2>(tS, dQh[h], dk_k0 + slot * kTileStep, idesc_k, h == 0 ? 0u : 1u);
         }                                     // the K halves stay: the dQ contractions read them again
-        if (ok) mma_commit(bar_sdp);
+        if (ok && leader) mma_commit(bar_sdp);
       };
       if (ok) {
         tc_fence_after();
@@ -213,20 +215,20 @@ bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       }
       for (int j = 0; ok && j < n_t; ++j) {
         if (j + 1 < n_t) {
-          if (!(ok = mbar_wait(bar_sfree, j & 1, &abort_flag, prm.status, BAR_SFREE))) break;
+          if (!(ok = mbar_wait_warp(bar_sfree, j & 1, &abort_flag, prm.status, BAR_SFREE))) break;
           tc_fence_after();
           issue_sdp(j + 1);
           if (!ok) break;
         }
-        if (!(ok = mbar_wait(bar_ds, j & 1, &abort_flag, prm.status, BAR_DS))) break;
+        if (!(ok = mbar_wait_warp(bar_ds, j & 1, &abort_flag, prm.status, BAR_DS))) break;
         tc_fence_after();
         for (int h = 0; h < nh; ++h) {                     // dQ_h += dS K_h over the 128 keys (eight K-steps)
           const int slot = (2 * j + h) % kDqKSlots;
-          mma_ts_x4<8, 128>(tdQ + 64 * h, tDS, dk_mn0 + slot * kTileStep, idesc_mn, j == 0 ? 0u : 1u);
-          mma_ts_x4<8, 128>(tdQ + 64 * h, tDS + 32, dk_mn0 + slot * kTileStep + 512, idesc_mn, 1u);
-          mma_commit(bar_kfree(slot));
+          if (leader) mma_ts_x4<8, 128>(tdQ + 64 * h, tDS, dk_mn0 + slot * kTileStep, idesc_mn, j == 0 ? 0u : 1u);
+          if (leader) mma_ts_x4<8, 128>(tdQ + 64 * h, tDS + 32, dk_mn0 + slot * kTileStep + 512, idesc_mn, 1u);
+          if (leader) mma_commit(bar_kfree(slot));
         }
-        mma_commit(bar_dq);                   // dS may be overwritten
+        if (leader) mma_commit(bar_dq);                   // dS may be overwritten
       }
     }
   } else {
@@ -254,7 +256,7 @@ bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           prefetch_l2(bn + 31 * prm.bsk);
         }
       }
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_sdp, j & 1, &abort_flag, prm.status, BAR_SDP))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_sdp, j & 1, &abort_flag, prm.status, BAR_SDP)) { alive = false; break; }
       tc_fence_after();
       uint32_t pk[16];
       {
@@ -323,7 +325,7 @@ bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       }
       if (j > 0) {
         // the dQ contractions of the previous key tile have read dS
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_dq, (j - 1) & 1, &abort_flag, prm.status, BAR_ACC))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_dq, (j - 1) & 1, &abort_flag, prm.status, BAR_ACC)) { alive = false; break; }
         tc_fence_after();
       }
       tmem_st16(tDS + lane_off + 16 * cq, pk);
@@ -335,7 +337,7 @@ bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
 #pragma unroll
     for (int i = 0; i < 16; ++i) { r0[i] = 0u; r1[i] = 0u; }
     if (alive && n_t > 0) {
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_dq, (n_t - 1) & 1, &abort_flag, prm.status, BAR_ACC))) alive = false;
+      if (!mbar_wait_warp(bar_dq, (n_t - 1) & 1, &abort_flag, prm.status, BAR_ACC)) alive = false;
       if (alive) {
         tc_fence_after();
         tmem_ld16(tdQ + lane_off + 16 * cq, r0);
@@ -376,6 +378,7 @@ bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __shared__ int abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.y;
   const int bi = bh / prm.heads, hi = bh - bi * prm.heads;   // tensor-map coordinates of this (batch*head)
   const int k0 = blockIdx.x * 128;                  // first (local) key row of this CTA
@@ -450,8 +453,9 @@ bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
       }
     }
-  } else if (warp == kIssuerWarp) {
-    if (n_it > 0 && lane == 0) {
+  } else if (warp_u == kIssuerWarp) {
+    if (n_it > 0) {
+      const bool leader = elect_one();
       // ---------------- MMA issuer ----------------
       constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
       constexpr uint32_t idesc_k = make_idesc(fmt, 0, 0, 128, 64);    // S^T, dP^T: A, B K-major, N = 64 queries
@@ -460,21 +464,21 @@ bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const uint64_t dVh[2] = {make_sdesc(sV(0), 16, 1024), make_sdesc(sV(1), 16, 1024)};
       const uint64_t dk_slot0 = make_sdesc(sSlot(0), 16, 1024), dmn_slot0 = make_sdesc(sSlot(0), 64 * 128, 1024);
       const int nh = BIAS ? prm.n_halves : 2;
-      bool ok = mbar_wait(bar_kv, 0, &abort_flag, prm.status, BAR_STAGE);
+      bool ok = mbar_wait_warp(bar_kv, 0, &abort_flag, prm.status, BAR_STAGE);
       auto issue_sdp = [&](int it) {
         for (int h = 0; h < nh && ok; ++h) {               // dP^T = sum over the halves of V_h dO_h^T
           const int seq = 2 * nh * it + h, slot = seq % kKvSlots;
-          if (!(ok = mbar_wait(bar_full(slot), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
+          if (!(ok = mbar_wait_warp(bar_full(slot), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
-          mma_ss_x4<2, 2>(tdP, dVh[h], dk_slot0 + slot * kSlotStep, idesc_k, h == 0 ? 0u : 1u);
+          if (leader) mma_ss_x4<2, 2>(tdP, dVh[h], dk_slot0 + slot * kSlotStep, idesc_k, h == 0 ? 0u : 1u);
         }
         for (int h = 0; h < nh && ok; ++h) {               // S^T = sum over the halves of K_h Q_h^T
           const int seq = 2 * nh * it + nh + h, slot = seq % kKvSlots;
-          if (!(ok = mbar_wait(bar_full(slot), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
+          if (!(ok = mbar_wait_warp(bar_full(slot), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
-          mma_ss_x4<2, 2>(tS, dKh[h], dk_slot0 + slot * kSlotStep, idesc_k, h == 0 ? 0u : 1u);
+          if (leader) mma_ss_x4<2, 2>(tS, dKh[h], dk_slot0 + slot * kSlotStep, idesc_k, h == 0 ? 0u : 1u);
         }
-        if (ok) mma_commit(bar_sdp);
+        if (ok && leader) mma_commit(bar_sdp);
       };
       if (ok) {
         tc_fence_after();
@@ -482,25 +486,25 @@ bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       for (int it = 0; ok && it < n_it; ++it) {
         if (it + 1 < n_it) {
-          if (!(ok = mbar_wait(bar_sfree, it & 1, &abort_flag, prm.status, BAR_SFREE))) break;
+          if (!(ok = mbar_wait_warp(bar_sfree, it & 1, &abort_flag, prm.status, BAR_SFREE))) break;
           tc_fence_after();
           issue_sdp(it + 1);
           if (!ok) break;
         }
-        if (!(ok = mbar_wait(bar_pl, it & 1, &abort_flag, prm.status, BAR_DS))) break;
+        if (!(ok = mbar_wait_warp(bar_pl, it & 1, &abort_flag, prm.status, BAR_DS))) break;
         tc_fence_after();
         const uint32_t acc = it == 0 ? 0u : 1u;
         for (int h = 0; h < nh; ++h) {                     // dV_h += P^T dO_h (64 queries: four K-steps)
           const int slot = (2 * nh * it + h) % kKvSlots;
-          mma_ts_x4<8, 128>(tdV + 64 * h, tP, dmn_slot0 + slot * kSlotStep, idesc_mn, acc);
-          mma_commit(bar_free(slot));
+          if (leader) mma_ts_x4<8, 128>(tdV + 64 * h, tP, dmn_slot0 + slot * kSlotStep, idesc_mn, acc);
+          if (leader) mma_commit(bar_free(slot));
         }
         for (int h = 0; h < nh; ++h) {                     // dK_h += dS^T Q_h
           const int slot = (2 * nh * it + nh + h) % kKvSlots;
-          mma_ts_x4<8, 128>(tdK + 64 * h, tDS, dmn_slot0 + slot * kSlotStep, idesc_mn, acc);
-          mma_commit(bar_free(slot));
+          if (leader) mma_ts_x4<8, 128>(tdK + 64 * h, tDS, dmn_slot0 + slot * kSlotStep, idesc_mn, acc);
+          if (leader) mma_commit(bar_free(slot));
         }
-        mma_commit(bar_acc);                  // P^T / dS^T may be overwritten
+        if (leader) mma_commit(bar_acc);                  // P^T / dS^T may be overwritten
       }
     }
   } else {
@@ -526,12 +530,12 @@ bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const int qn = q_tile0 + 64 + 16 * cq + (lane & 15);
         if (it + 1 < n_it && qn < N) prefetch_l2(bias_col + static_cast<int64_t>(qn) * prm.bsq);
       }
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_sdp, it & 1, &abort_flag, prm.status, BAR_SDP))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_sdp, it & 1, &abort_flag, prm.status, BAR_SDP)) { alive = false; break; }
       // the tile's row statistics were written by the bulk copies that complete on its first slot's barrier: observe
       // that barrier directly (it completed before the MMAs behind bar_sdp were issued, so this never spins)
       {
         const int seq = 2 * n_halves * it;
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_full(seq % kKvSlots), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_full(seq % kKvSlots), (seq / kKvSlots) & 1, &abort_flag, prm.status, BAR_FULL)) { alive = false; break; }
       }
       tc_fence_after();
       uint32_t pk[8], dsk[8];
@@ -578,7 +582,7 @@ bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       if (it > 0) {
         // the dV / dK contractions of the previous query tile have read P^T and dS^T
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_acc, (it - 1) & 1, &abort_flag, prm.status, BAR_ACC))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_acc, (it - 1) & 1, &abort_flag, prm.status, BAR_ACC)) { alive = false; break; }
         tc_fence_after();
       }
       tmem_st8(tP + lane_off + 8 * cq, pk);
@@ -587,7 +591,7 @@ bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       tc_fence_before();
       mbar_arrive_warp(bar_pl, lane);
     }
-    if (alive && n_it > 0 && !__all_sync(0xffffffffu, mbar_wait(bar_acc, (n_it - 1) & 1, &abort_flag, prm.status, BAR_ACC))) alive = false;
+    if (alive && n_it > 0 && !mbar_wait_warp(bar_acc, (n_it - 1) & 1, &abort_flag, prm.status, BAR_ACC)) alive = false;
     if (alive) {
       // dK, dV of this key tile (tcgen05.ld is warp-collective: only the stores are predicated)
       const int d = prm.head_dim;

@@ -25,6 +25,12 @@
 // max is tracked separately and the summary is renormalised to it in the epilogue, so the stored
 // (m, z, s) is the same monoid element the FP32-FMA kernel produces.
 //
+// Two changes took (1,8,16384,64) fp16 from 0.700 to 0.659 ms, causal bf16 from 0.407 to 0.383, (8,3,4097,64) from 0.173
+// to 0.157 and (64,3,197,64) from 20.5 to 18.6 us: the issuing warps run warp-uniform code (elect_one in tc_common.cuh),
+// and tile 1 starts half a period after tile 0.  Cycles per key tile and row: exponentials and P stores 1290 (1165 with
+// the ex2 unit to itself), waits, TMEM loads and the maximum 1030; the period of a tile is 2565, so the ex2 unit is at
+// 80 %.  Every n-th pair of exponentials on the FMA pipe (n = 4, 8, 16) gains nothing at this point.
+//
 // Measured alternatives at B=1 H=8 N=16384 (this design: 0.738 ms; with a P hand-off per 64-key half 0.755 ms and
 // the variants below were measured against that): two threads per row (four fold
 // warpgroups of 64 columns each, half-row max exchanged through shared memory) 0.77-0.79 ms; a fixed
@@ -95,11 +101,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 fold_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                const __grid_constant__ CUtensorMap tmap_v, const FoldTcParams prm) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[2 * kStages + 11];   // q, kv_full x4, kv_free x4, then 5 pairs
+  __shared__ __align__(8) uint64_t bars[2 * kStages + 12];   // q, kv_full x4, kv_free x4, 5 pairs, stagger
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.z, part = blockIdx.y;
   const int bi = bh / prm.heads, hi = bh - bi * prm.heads;  // tensor-map coordinates of this (batch*head)
   // causal: a tile's work grows with its first row, so the tiles are handed out from the last one down -- the long
@@ -136,15 +143,18 @@ fold_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   auto bar_sfree = [&](int t) { return bar0 + 8 * (7 + 2 * kStages + t); };      // the fold warps hold S_t in registers
   auto bar_pv = [&](int t) { return bar0 + 8 * (9 + 2 * kStages + t); };         // P_t V of the current key tile has retired
 
+  const uint32_t bar_stagger = bar0 + 8 * (11 + 2 * kStages);                    // tile 1 may start
+
   if (tid == 0) {
     abort_flag = 0;
     mbar_init(bar_q, 1);
+    mbar_init(bar_stagger, 1);
     // a K/V stage is free again when BOTH tiles' issuers have released it (a commit after the tile's P V, or a plain
     // arrival for a key tile that the tile does not visit)
     for (int st = 0; st < kStages; ++st) { mbar_init(bar_kv_full(st), 1); mbar_init(bar_kv_free(st), 2); }
     for (int t = 0; t < 2; ++t) {
-      mbar_init(bar_s(t), 1); mbar_init(bar_p(t), 128); mbar_init(bar_o(t), 1);
-      mbar_init(bar_sfree(t), 128); mbar_init(bar_pv(t), 1);
+      mbar_init(bar_s(t), 1); mbar_init(bar_p(t), 4); mbar_init(bar_o(t), 1);
+      mbar_init(bar_sfree(t), 4); mbar_init(bar_pv(t), 1);
     }
     fence_mbar_init();
   }
@@ -164,7 +174,7 @@ fold_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   // warpgroup needs almost nothing (3 x 128 threads: 232 + 232 + 40 = 3 x 168, the launch allocation; setmaxnreg.inc waits, unbounded, until the pool has the registers, so the three budgets must never add up to more).  Each role
   // branch starts with its setmaxnreg and runs to the common exit, so the allocator sees one budget per branch.
 
-  if (warp >= 8) {
+  if (warp_u >= 8) {
     reg_dec<40>();
     if (n_max > 0 && warp == kProducerWarp) {
       // ---------------- TMA producer ----------------
@@ -181,14 +191,15 @@ fold_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           tma_load_4d(sV(st), &tmap_v, bar_kv_full(st), 0, k_begin + j * 128, hi, bi);
         }
       }
-    } else if (n_max > 0 && (warp == kIssuerWarp || warp == kIssuerWarp + 1)) {
+    } else if (n_max > 0 && (warp_u == kIssuerWarp || warp_u == kIssuerWarp + 1)) {
       // ---------------- MMA issuers: one thread per query tile ----------------
       // Each tile has its own issuing thread, so the two tiles run their chains (scores -> exponentials -> P V)
       // independently and drift half a period apart by themselves: while one tile's P V and hand-offs are in
       // flight, the other tile's fold warps have the ex2 unit to themselves.  The only thing the tiles share is
       // the K/V ring (and the tensor pipe, which executes the MMAs of both threads in the order it receives them).
-      const int t = warp - kIssuerWarp;
-      if (lane == 0) {
+      const int t = warp_u - kIssuerWarp;
+      const bool leader = elect_one();
+      {
         constexpr uint32_t fmt = sizeof(T) == 2 && std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
         constexpr uint32_t idesc_s = make_idesc(fmt, 0, 0, 128, 128);   // S = Q K^T : A, B K-major
         constexpr uint32_t idesc_o = make_idesc(fmt, 0, 1, 128, 64);    // O += P V  : A in TMEM, B (V) MN-major
@@ -199,11 +210,14 @@ fold_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         const int nt = n_t[t];
         bool ok = true;
         if (nt > 0) {
-          ok = mbar_wait(bar_q, 0, &abort_flag, prm.status, BAR_Q) && mbar_wait(bar_kv_full(0), 0, &abort_flag, prm.status, BAR_KV_FULL);
+          ok = mbar_wait_warp(bar_q, 0, &abort_flag, prm.status, BAR_Q) && mbar_wait_warp(bar_kv_full(0), 0, &abort_flag, prm.status, BAR_KV_FULL);
+          // tile 1 starts half a period after tile 0: two tiles in step would want the ex2 unit at the same time and leave
+          // it idle at the same time, and nothing later moves them apart
+          if (ok && t == 1 && n_t[0] > 0) ok = mbar_wait_warp(bar_stagger, 0, &abort_flag, prm.status, BAR_S);
           if (ok) {
             tc_fence_after();
-            mma_ss_x4<2, 2>(tS[t], dq, dk0, idesc_s, 0u);
-            mma_commit(bar_s(t));
+            if (leader) mma_ss_x4<2, 2>(tS[t], dq, dk0, idesc_s, 0u);
+            if (leader) mma_commit(bar_s(t));
           }
         }
         for (int j = 0; ok && j < nt; ++j) {
@@ -211,28 +225,29 @@ fold_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           // S(j+1) as soon as the fold warps have pulled S(j) into registers: the next scores are computed while
           // the current exponentials run, so the fold warps never wait for the tensor pipe
           if (j + 1 < nt) {
-            ok = mbar_wait(bar_kv_full(un), ((j + 1) / kStages) & 1, &abort_flag, prm.status, BAR_KV_FULL) &&
-                 mbar_wait(bar_sfree(t), j & 1, &abort_flag, prm.status, BAR_SFREE);
+            ok = mbar_wait_warp(bar_kv_full(un), ((j + 1) / kStages) & 1, &abort_flag, prm.status, BAR_KV_FULL) &&
+                 mbar_wait_warp(bar_sfree(t), j & 1, &abort_flag, prm.status, BAR_SFREE);
             if (!ok) break;
             tc_fence_after();
-            mma_ss_x4<2, 2>(tS[t], dq, dk0 + un * kStageStep, idesc_s, 0u);
-            mma_commit(bar_s(t));
+            if (leader) mma_ss_x4<2, 2>(tS[t], dq, dk0 + un * kStageStep, idesc_s, 0u);
+            if (leader) mma_commit(bar_s(t));
           }
+          if (t == 0 && j == 0 && leader) mbar_arrive(bar_stagger);
           // O += P V once the fold warps have delivered P(j)
-          if (!(ok = mbar_wait(bar_p(t), j & 1, &abort_flag, prm.status, BAR_P))) break;
+          if (!(ok = mbar_wait_warp(bar_p(t), j & 1, &abort_flag, prm.status, BAR_P))) break;
           tc_fence_after();
-          mma_ts_x4<8, 128>(tO[t], tP[t], dv0 + u * kStageStep, idesc_o, j > 0 ? 1u : 0u);
-          mma_ts_x4<8, 128>(tO[t], tP[t] + 32, dv0 + u * kStageStep + 512, idesc_o, 1u);
-          mma_commit(bar_pv(t));        // P_t may be overwritten, O_t may be rescaled
-          mma_commit(bar_kv_free(u));   // this tile no longer reads K(j), V(j)
+          if (leader) mma_ts_x4<8, 128>(tO[t], tP[t], dv0 + u * kStageStep, idesc_o, j > 0 ? 1u : 0u);
+          if (leader) mma_ts_x4<8, 128>(tO[t], tP[t] + 32, dv0 + u * kStageStep + 512, idesc_o, 1u);
+          if (leader) mma_commit(bar_pv(t));        // P_t may be overwritten, O_t may be rescaled
+          if (leader) mma_commit(bar_kv_free(u));   // this tile no longer reads K(j), V(j)
         }
-        if (ok && nt > 0) mma_commit(bar_o(t));
+        if (ok && nt > 0 && leader) mma_commit(bar_o(t));
         // key tiles this query tile does not visit (causal: the other tile reaches one tile further; a tile beyond
         // the last query row visits none): release their stages in order, each after the stage's previous use is over
         for (int j = nt; ok && j < n_max; ++j) {
           const int u = j % kStages;
-          if (j >= kStages && !(ok = mbar_wait(bar_kv_free(u), ((j / kStages) - 1) & 1, &abort_flag, prm.status, BAR_KV_FREE))) break;
-          mbar_arrive(bar_kv_free(u));
+          if (j >= kStages && !(ok = mbar_wait_warp(bar_kv_free(u), ((j / kStages) - 1) & 1, &abort_flag, prm.status, BAR_KV_FREE))) break;
+          if (leader) mbar_arrive(bar_kv_free(u));
         }
       }
     }
@@ -248,48 +263,59 @@ fold_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     bool alive = true;
 
     for (int j = 0; j < n_t[t]; ++j) {
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_s(t), j & 1, &abort_flag, prm.status, BAR_S))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_s(t), j & 1, &abort_flag, prm.status, BAR_S)) { alive = false; break; }
       tc_fence_after();
+      // the scores in two halves: the maximum of the first is taken while the second is on its way out of TMEM
       float sv[128];
+      float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+      {
+        uint32_t ra[32], rb[32], rc[32], rd[32];
+        tmem_ld32(tS[t] + lane_off, ra);
+        tmem_ld32(tS[t] + lane_off + 32, rb);
+        tmem_wait_ld();
+        tmem_ld32(tS[t] + lane_off + 64, rc);
+        tmem_ld32(tS[t] + lane_off + 96, rd);
 #pragma unroll
-      for (int cchunk = 0; cchunk < 4; ++cchunk) {
-        uint32_t r[32];
-        tmem_ld32(tS[t] + lane_off + 32 * cchunk, r);
+        for (int i = 0; i < 32; ++i) { sv[i] = __uint_as_float(ra[i]); sv[32 + i] = __uint_as_float(rb[i]); }
+        // (four independent chains of three-input maxima)
 #pragma unroll
-        for (int i = 0; i < 32; ++i) sv[32 * cchunk + i] = __uint_as_float(r[i]);
+        for (int i = 0; i < 64; i += 8) {
+          mx[0] = max3(mx[0], sv[i], sv[i + 1]); mx[1] = max3(mx[1], sv[i + 2], sv[i + 3]);
+          mx[2] = max3(mx[2], sv[i + 4], sv[i + 5]); mx[3] = max3(mx[3], sv[i + 6], sv[i + 7]);
+        }
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive_warp(bar_sfree(t), lane);      // S_t may be overwritten with the next tile's scores
+#pragma unroll
+        for (int i = 0; i < 32; ++i) { sv[64 + i] = __uint_as_float(rc[i]); sv[96 + i] = __uint_as_float(rd[i]); }
+#pragma unroll
+        for (int i = 64; i < 128; i += 8) {
+          mx[0] = max3(mx[0], sv[i], sv[i + 1]); mx[1] = max3(mx[1], sv[i + 2], sv[i + 3]);
+          mx[2] = max3(mx[2], sv[i + 4], sv[i + 5]); mx[3] = max3(mx[3], sv[i + 6], sv[i + 7]);
+        }
       }
-      tmem_wait_ld();
-      tc_fence_before();
-      mbar_arrive(bar_sfree(t));      // S_t may be overwritten with the next tile's scores
       const int k0 = k_begin + j * 128;
       const bool tail = k0 + 128 > k_end;
       const bool diag = prm.is_causal && (k0 + koff + 127 > q0 + t * 128);
-      if (tail || diag) {
+      if (__builtin_expect(tail || diag, 0)) {
         const int lim = prm.is_causal ? min(k_end - 1, qi - koff) : k_end - 1;   // last admissible (local) key of this row
+        mx[0] = mx[1] = mx[2] = mx[3] = -CUDART_INF_F;
 #pragma unroll
-        for (int i = 0; i < 128; ++i)
+        for (int i = 0; i < 128; ++i) {
           if (k0 + i > lim) sv[i] = -CUDART_INF_F;
+          mx[i & 3] = fmaxf(mx[i & 3], sv[i]);
+        }
       }
-      // row max with four independent chains (a single 128-deep fmax chain costs ~500 cycles of latency)
-      // (three-input max: 64 instructions instead of 128)
-      float mx[4] = {sv[0], sv[1], sv[2], sv[3]};
-#pragma unroll
-      for (int i = 4; i < 124; i += 8) {
-        mx[0] = max3(mx[0], sv[i], sv[i + 1]); mx[1] = max3(mx[1], sv[i + 2], sv[i + 3]);
-        mx[2] = max3(mx[2], sv[i + 4], sv[i + 5]); mx[3] = max3(mx[3], sv[i + 6], sv[i + 7]);
-      }
-      mx[0] = max3(mx[0], sv[124], sv[125]);
-      mx[1] = max3(mx[1], sv[126], sv[127]);
       float tmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       tmax *= c;
       m_true = fmaxf(m_true, tmax);
       if (j > 0) {
         // P_t V of the previous key tile must have retired before P_t is overwritten or O_t rescaled
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_pv(t), (j - 1) & 1, &abort_flag, prm.status, BAR_PV))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_pv(t), (j - 1) & 1, &abort_flag, prm.status, BAR_PV)) { alive = false; break; }
         tc_fence_after();
       }
       const bool move = tmax > m_ref + kRescaleThreshold;   // also true for the first admissible tile (m_ref = -inf)
-      if (__any_sync(0xffffffffu, move)) {
+      if (__builtin_expect(__any_sync(0xffffffffu, move), 0)) {
         const float m_new = fmaxf(m_ref, tmax);
         const float alpha = (m_new == -CUDART_INF_F) ? 1.f : fast_exp2(m_ref - m_new);
         zsum *= alpha;
@@ -325,7 +351,7 @@ fold_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       // one hand-off per key tile: with the scores produced a tile ahead, P V need not start on the first half
       tmem_wait_st();               // (also covers the O rescale stores above)
       tc_fence_before();
-      mbar_arrive(bar_p(t));
+      mbar_arrive_warp(bar_p(t), lane);
       {
         const float2 s01 = __fadd2_rn(ps[0], ps[1]), s23 = __fadd2_rn(ps[2], ps[3]);
         const float2 s = __fadd2_rn(s01, s23);
@@ -337,7 +363,7 @@ fold_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     const int r_chunk = bx * 256 + t * 128 + row;   // row within the query chunk
     const bool row_ok = r_chunk < prm.q_len;
     if (n_t[t] > 0) {
-      if (alive && !__all_sync(0xffffffffu, mbar_wait(bar_o(t), 0, &abort_flag, prm.status, BAR_O))) alive = false;
+      if (alive && !mbar_wait_warp(bar_o(t), 0, &abort_flag, prm.status, BAR_O)) alive = false;
       if (alive) {
         tc_fence_after();
         float ov[64];

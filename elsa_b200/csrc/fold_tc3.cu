@@ -195,6 +195,7 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __shared__ float row_sum[4][128];      // the quarter-row sums, exchanged once in the epilogue
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.z, part = blockIdx.y;
   // causal: a tile's work grows with its first row, so the tiles are handed out from the last one down -- the long
   // ones first, the short ones fill the end of the last wave
@@ -264,8 +265,9 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         for (int p = kPlanes - 1; p >= 0 && ok; --p) load(&tmap_v, j, p);
       }
     }
-  } else if (warp == kIssuerWarp) {
-    if (n_t > 0 && lane == 0) {
+  } else if (warp_u == kIssuerWarp) {
+    if (n_t > 0) {
+      const bool leader = elect_one();
       // ---------------- MMA issuer ----------------
       constexpr uint32_t idesc_s = make_idesc(kPlaneFmt, 0, 0, 128, 128);   // S += Qp Kp^T : bf16, A, B K-major
       constexpr uint32_t idesc_o = make_idesc(kPlaneFmt, 0, 1, 128, 64);    // O += Pp Vp   : A in TMEM, B (V) MN-major
@@ -274,52 +276,52 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const uint64_t dk_slot0 = make_sdesc(sSlot(0), 16, 1024), dv_slot0 = make_sdesc(sSlot(0), 128 * 128, 1024);
       constexpr uint64_t kSlotStep = kPlaneBytes >> 4;   // descriptor address field counts 16-byte units
       int seq = 0;
-      bool ok = mbar_wait(bar_q, 0, &abort_flag, prm.status, BAR_Q);
+      bool ok = mbar_wait_warp(bar_q, 0, &abort_flag, prm.status, BAR_Q);
       // the six (q plane, k plane) pairs of one key tile; K planes arrive in ring order 2, 1, 0 and within a plane
       // the q planes go from the lightest admissible one down to q0: the leading term q0 k0 is the last to be added
       auto issue_s = [&]() {
         bool first = true;
         for (int kp = kPlanes - 1; kp >= 0 && ok; --kp) {
           const int slot = seq % kSlots;
-          if (!(ok = mbar_wait(bar_full(slot), (seq / kSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
+          if (!(ok = mbar_wait_warp(bar_full(slot), (seq / kSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
           const uint64_t dk = dk_slot0 + slot * kSlotStep;
           for (int qp = kPlanes - 1 - kp; qp >= 0; --qp) {
-            mma_ss_x4<2, 2>(tS, dq[qp], dk, idesc_s, first ? 0u : 1u);
+            if (leader) mma_ss_x4<2, 2>(tS, dq[qp], dk, idesc_s, first ? 0u : 1u);
             first = false;
           }
-          mma_commit(bar_free(slot));     // the plane tile is free again once these MMAs have retired
+          if (leader) mma_commit(bar_free(slot));     // the plane tile is free again once these MMAs have retired
           ++seq;
         }
-        if (ok) mma_commit(bar_s);
+        if (ok && leader) mma_commit(bar_s);
       };
       if (ok) issue_s();
       for (int j = 0; ok && j < n_t; ++j) {
         if (j + 1 < n_t) {
           // S(j+1) as soon as the fold warps hold S(j) in registers: it runs while they work on tile j
-          if (!(ok = mbar_wait(bar_sfree, j & 1, &abort_flag, prm.status, BAR_SFREE))) break;
+          if (!(ok = mbar_wait_warp(bar_sfree, j & 1, &abort_flag, prm.status, BAR_SFREE))) break;
           tc_fence_after();
           issue_s();
           if (!ok) break;
         }
-        if (!(ok = mbar_wait(bar_p, j & 1, &abort_flag, prm.status, BAR_P))) break;
+        if (!(ok = mbar_wait_warp(bar_p, j & 1, &abort_flag, prm.status, BAR_P))) break;
         tc_fence_after();
         // O_j starts from zero (the fold warps took O_{j-1} into their registers before they delivered P(j))
         bool first = true;
         for (int vp = kPlanes - 1; vp >= 0 && ok; --vp) {
           const int slot = seq % kSlots;
-          if (!(ok = mbar_wait(bar_full(slot), (seq / kSlots) & 1, &abort_flag, prm.status, BAR_FULL))) break;
+          if (!(ok = mbar_wait_warp(bar_full(slot), (seq / kSlots) & 1, &abort_flag, prm.status, BAR_FULL))) break;
           tc_fence_after();
           const uint64_t dv = dv_slot0 + slot * kSlotStep;
           for (int pp = kPlanes - 1 - vp; pp >= 0; --pp) {
-            mma_ts_x4<8, 128>(tO, tP0 + 64 * pp, dv, idesc_o, first ? 0u : 1u);
-            mma_ts_x4<8, 128>(tO, tP0 + 64 * pp + 32, dv + 512, idesc_o, 1u);
+            if (leader) mma_ts_x4<8, 128>(tO, tP0 + 64 * pp, dv, idesc_o, first ? 0u : 1u);
+            if (leader) mma_ts_x4<8, 128>(tO, tP0 + 64 * pp + 32, dv + 512, idesc_o, 1u);
             first = false;
           }
-          mma_commit(bar_free(slot));
+          if (leader) mma_commit(bar_free(slot));
           ++seq;
         }
-        if (ok) mma_commit(bar_pv);      // O_j is complete; the P planes may be overwritten
+        if (ok && leader) mma_commit(bar_pv);      // O_j is complete; the P planes may be overwritten
       }
     }
   } else {
@@ -353,7 +355,7 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     };
 
     for (int j = 0; j < n_t; ++j) {
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_s, j & 1, &abort_flag, prm.status, BAR_S))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_s, j & 1, &abort_flag, prm.status, BAR_S)) { alive = false; break; }
       tc_fence_after();
       float sv[32];
       {
@@ -403,7 +405,7 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       mx[0] = max3f(mx[0], sv[28], sv[29]); mx[1] = max3f(mx[1], sv[30], sv[31]);
       row_max[j & 1][cq][row] = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       mbar_arrive_warp(bar_row(qd), lane);
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_row(qd), j & 1, &abort_flag, prm.status, BAR_ROW))) { alive = false; break; }
+      if (!mbar_wait_warp(bar_row(qd), j & 1, &abort_flag, prm.status, BAR_ROW)) { alive = false; break; }
       float tmax = fmaxf(fmaxf(row_max[j & 1][0][row], row_max[j & 1][1][row]), fmaxf(row_max[j & 1][2][row], row_max[j & 1][3][row]));
       tmax *= cc;
       m_true = fmaxf(m_true, tmax);
@@ -431,7 +433,7 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (j > 0) {
         // P V of the previous key tile has retired: its O goes into the running sum (both are relative to the m_ref
         // of that tile) before P V of this tile starts the accumulator from zero again; the P planes are free
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_pv, (j - 1) & 1, &abort_flag, prm.status, BAR_PV))) { alive = false; break; }
+        if (!mbar_wait_warp(bar_pv, (j - 1) & 1, &abort_flag, prm.status, BAR_PV)) { alive = false; break; }
         tc_fence_after();
         take_o();
       }
@@ -464,13 +466,13 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const int64_t ro = (static_cast<int64_t>(part) * prm.bh + bh) * prm.q_len + r_chunk;
     float m_out = -CUDART_INF_F, z_out = 0.f;
     if (n_t > 0) {
-      if (alive && !__all_sync(0xffffffffu, mbar_wait(bar_pv, (n_t - 1) & 1, &abort_flag, prm.status, BAR_O))) alive = false;
+      if (alive && !mbar_wait_warp(bar_pv, (n_t - 1) & 1, &abort_flag, prm.status, BAR_O)) alive = false;
       if (alive) {
         tc_fence_after();
         take_o();
         row_sum[cq][row] = zsum;
         mbar_arrive_warp(bar_row(qd), lane);
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_row(qd), n_t & 1, &abort_flag, prm.status, BAR_ROW))) alive = false;
+        if (!mbar_wait_warp(bar_row(qd), n_t & 1, &abort_flag, prm.status, BAR_ROW)) alive = false;
       }
       if (alive) {
         const float ztot = (row_sum[0][row] + row_sum[1][row]) + (row_sum[2][row] + row_sum[3][row]);

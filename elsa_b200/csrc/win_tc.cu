@@ -78,6 +78,7 @@ win_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   __shared__ int abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int b0 = blockIdx.x * 2, hi = blockIdx.y;
   const int N = prm.n_ctx, d = prm.head_dim;
 
@@ -101,32 +102,33 @@ win_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const uint32_t tmem_base = tmem_base_slot;
   const uint32_t tS = tmem_base, tO = tmem_base + 128, tP = tmem_base + 192;
 
-  if (warp == 4) {
-    if (lane == 0) {
+  if (warp_u == 4) {
+    {
+      const bool leader = elect_one();
       // ---------------- loads and MMAs ----------------
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
-      mbar_arrive_expect_tx(bar_load, 3 * kTileBytes);
-      tma_load_4d(sQ, &tmap_q, bar_load, 0, 0, hi, b0);     // rows beyond N, columns beyond d, a batch entry beyond B: zeros
-      tma_load_4d(sK, &tmap_k, bar_load, 0, 0, hi, b0);
-      tma_load_4d(sV, &tmap_v, bar_load, 0, 0, hi, b0);
+      if (leader) mbar_arrive_expect_tx(bar_load, 3 * kTileBytes);
+      if (leader) tma_load_4d(sQ, &tmap_q, bar_load, 0, 0, hi, b0);     // rows beyond N, columns beyond d, a batch entry beyond B: zeros
+      if (leader) tma_load_4d(sK, &tmap_k, bar_load, 0, 0, hi, b0);
+      if (leader) tma_load_4d(sV, &tmap_v, bar_load, 0, 0, hi, b0);
       constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
       constexpr uint32_t idesc_s = make_idesc(fmt, 0, 0, 128, 128);   // S = Q K^T : A, B K-major
       constexpr uint32_t idesc_o = make_idesc(fmt, 0, 1, 128, 64);    // O = P V   : A in TMEM, B (V) MN-major
-      bool ok = mbar_wait(bar_load, 0, &abort_flag, prm.status, BAR_LOAD);
+      bool ok = mbar_wait_warp(bar_load, 0, &abort_flag, prm.status, BAR_LOAD);
       if (ok) {
         tc_fence_after();
         const uint64_t dq = make_sdesc(sQ, 16, 1024), dk = make_sdesc(sK, 16, 1024);
         const int ksteps = (d + 15) / 16;                     // the columns beyond d are zeros: their K-steps add nothing
-        for (int ks = 0; ks < ksteps; ++ks) mma_ss(tS, dq + 2 * ks, dk + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
-        mma_commit(bar_s);
-        ok = mbar_wait(bar_p, 0, &abort_flag, prm.status, BAR_P);
+        for (int ks = 0; ks < ksteps; ++ks) if (leader) mma_ss(tS, dq + 2 * ks, dk + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+        if (leader) mma_commit(bar_s);
+        ok = mbar_wait_warp(bar_p, 0, &abort_flag, prm.status, BAR_P);
       }
       if (ok) {
         tc_fence_after();
         const uint64_t dv = make_sdesc(sV, 128 * 128, 1024);
-        mma_ts_x4<8, 128>(tO, tP, dv, idesc_o, 0u);
-        mma_ts_x4<8, 128>(tO, tP + 32, dv + 512, idesc_o, 1u);
-        mma_commit(bar_o);
+        if (leader) mma_ts_x4<8, 128>(tO, tP, dv, idesc_o, 0u);
+        if (leader) mma_ts_x4<8, 128>(tO, tP + 32, dv + 512, idesc_o, 1u);
+        if (leader) mma_commit(bar_o);
       }
     }
   } else {
@@ -142,7 +144,7 @@ win_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       stage_bias(sb, prm.bias, prm.bsb, prm.bsh, prm.bsq, prm.bsk, b0, prm.bsb != 0 ? 2 : 1, prm.batch, hi, N, warp, 4, lane);
       named_barrier_sync(1, 128);
     }
-    bool alive = __all_sync(0xffffffffu, mbar_wait(bar_s, 0, &abort_flag, prm.status, BAR_S));
+    bool alive = mbar_wait_warp(bar_s, 0, &abort_flag, prm.status, BAR_S);
     float z = 0.f, m = -CUDART_INF_F;
     if (alive) {
       tc_fence_after();
@@ -193,7 +195,7 @@ win_tc_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive_warp(bar_p, lane);
-      alive = __all_sync(0xffffffffu, mbar_wait(bar_o, 0, &abort_flag, prm.status, BAR_O));
+      alive = mbar_wait_warp(bar_o, 0, &abort_flag, prm.status, BAR_O);
     }
     if (alive) {
       tc_fence_after();
@@ -325,6 +327,7 @@ win_tc_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   __shared__ float nlse_s[2][128], nd_s[2][128];   // -LSE and -D of the tile's 128 query rows, per iteration parity
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int hi = blockIdx.x % prm.heads;
   const int pair0 = blockIdx.x / prm.heads, pair_step = gridDim.x / prm.heads;
   const int n_pairs = (prm.batch + 1) / 2;
@@ -365,8 +368,9 @@ win_tc_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const bool bias_per_batch = prm.bias && prm.bsb != 0;   // else one tile serves every pair of this head
   const float* sb_seq = sb + (bias_per_batch ? seq * kBiasTile : 0);
 
-  if (warp == 16) {
-    if (lane == 0 && pair0 < n_pairs) {
+  if (warp_u == 16) {
+    if (pair0 < n_pairs) {
+      const bool leader = elect_one();
       // ---------------- loads and MMAs ----------------
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v); prefetch_tmap(&tmap_do); prefetch_tmap(&tmap_o);
       constexpr uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
@@ -375,12 +379,12 @@ win_tc_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const int ksteps = (d + 15) / 16;                     // the columns beyond d are zeros: their K-steps add nothing
       auto issue_loads = [&](int pair, int stage) {         // rows beyond N, columns beyond d, a batch entry beyond B: zeros
         const uint32_t base = smem_base + stage * kBwdStageBytes, bar = bar_load + 8 * stage;
-        mbar_arrive_expect_tx(bar, 5 * kTileBytes);
-        tma_load_4d(base, &tmap_q, bar, 0, 0, hi, 2 * pair);
-        tma_load_4d(base + kTileBytes, &tmap_k, bar, 0, 0, hi, 2 * pair);
-        tma_load_4d(base + 2 * kTileBytes, &tmap_v, bar, 0, 0, hi, 2 * pair);
-        tma_load_4d(base + 3 * kTileBytes, &tmap_do, bar, 0, 0, hi, 2 * pair);
-        tma_load_4d(base + 4 * kTileBytes, &tmap_o, bar, 0, 0, hi, 2 * pair);
+        if (leader) mbar_arrive_expect_tx(bar, 5 * kTileBytes);
+        if (leader) tma_load_4d(base, &tmap_q, bar, 0, 0, hi, 2 * pair);
+        if (leader) tma_load_4d(base + kTileBytes, &tmap_k, bar, 0, 0, hi, 2 * pair);
+        if (leader) tma_load_4d(base + 2 * kTileBytes, &tmap_v, bar, 0, 0, hi, 2 * pair);
+        if (leader) tma_load_4d(base + 3 * kTileBytes, &tmap_do, bar, 0, 0, hi, 2 * pair);
+        if (leader) tma_load_4d(base + 4 * kTileBytes, &tmap_o, bar, 0, 0, hi, 2 * pair);
       };
       issue_loads(pair0, 0);
       int it = 0;
@@ -388,34 +392,34 @@ win_tc_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         const int stage = it & 1;
         const uint32_t ph = it & 1;
         const uint32_t sQ = smem_base + stage * kBwdStageBytes, sK = sQ + kTileBytes, sV = sQ + 2 * kTileBytes, sDO = sQ + 3 * kTileBytes;
-        if (!mbar_wait(bar_load + 8 * stage, (it >> 1) & 1, &abort_flag, prm.status, BAR_BLOAD)) break;
+        if (!mbar_wait_warp(bar_load + 8 * stage, (it >> 1) & 1, &abort_flag, prm.status, BAR_BLOAD)) break;
         // the fold warps have read the gradients of the previous pair out of TMEM (and its tiles out of the other stage)
-        if (it > 0 && !mbar_wait(bar_epi, (it - 1) & 1, &abort_flag, prm.status, BAR_EPI)) break;
+        if (it > 0 && !mbar_wait_warp(bar_epi, (it - 1) & 1, &abort_flag, prm.status, BAR_EPI)) break;
         tc_fence_after();
         const uint64_t dq = make_sdesc(sQ, 16, 1024), dk = make_sdesc(sK, 16, 1024);
         const uint64_t dv = make_sdesc(sV, 16, 1024), ddo = make_sdesc(sDO, 16, 1024);
         // the key side has the longer way to go (two products, two gradients): its inputs first
-        for (int ks = 0; ks < ksteps; ++ks) mma_ss(tST, dk + 2 * ks, dq + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
-        for (int ks = 0; ks < ksteps; ++ks) mma_ss(tdPT, dv + 2 * ks, ddo + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
-        mma_commit(bar_r1k);
-        for (int ks = 0; ks < ksteps; ++ks) mma_ss(tS, dq + 2 * ks, dk + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
-        for (int ks = 0; ks < ksteps; ++ks) mma_ss(tdP, ddo + 2 * ks, dv + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
-        mma_commit(bar_r1);
+        for (int ks = 0; ks < ksteps; ++ks) if (leader) mma_ss(tST, dk + 2 * ks, dq + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < ksteps; ++ks) if (leader) mma_ss(tdPT, dv + 2 * ks, ddo + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+        if (leader) mma_commit(bar_r1k);
+        for (int ks = 0; ks < ksteps; ++ks) if (leader) mma_ss(tS, dq + 2 * ks, dk + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+        for (int ks = 0; ks < ksteps; ++ks) if (leader) mma_ss(tdP, ddo + 2 * ks, dv + 2 * ks, idesc_s, ks > 0 ? 1u : 0u);
+        if (leader) mma_commit(bar_r1);
         if (pair + pair_step < n_pairs) issue_loads(pair + pair_step, stage ^ 1);
         const uint64_t k_mn = make_sdesc(sK, 128 * 128, 1024), q_mn = make_sdesc(sQ, 128 * 128, 1024);
         const uint64_t do_mn = make_sdesc(sDO, 128 * 128, 1024);
-        if (!mbar_wait(bar_phq, ph, &abort_flag, prm.status, BAR_PHQ)) break;
+        if (!mbar_wait_warp(bar_phq, ph, &abort_flag, prm.status, BAR_PHQ)) break;
         tc_fence_after();
-        mma_ts_x4<8, 128>(tdP, tS, k_mn, idesc_o, 0u);                 // dQ = dS K
-        mma_ts_x4<8, 128>(tdP, tS + 32, k_mn + 512, idesc_o, 1u);
-        mma_commit(bar_r2q);
-        if (!mbar_wait(bar_phk, ph, &abort_flag, prm.status, BAR_PHK)) break;
+        if (leader) mma_ts_x4<8, 128>(tdP, tS, k_mn, idesc_o, 0u);                 // dQ = dS K
+        if (leader) mma_ts_x4<8, 128>(tdP, tS + 32, k_mn + 512, idesc_o, 1u);
+        if (leader) mma_commit(bar_r2q);
+        if (!mbar_wait_warp(bar_phk, ph, &abort_flag, prm.status, BAR_PHK)) break;
         tc_fence_after();
-        mma_ts_x4<8, 128>(tdPT, tST, do_mn, idesc_o, 0u);              // dV = P^T dO
-        mma_ts_x4<8, 128>(tdPT, tST + 32, do_mn + 512, idesc_o, 1u);
-        mma_ts_x4<8, 128>(tdPT + 64, tST + 64, q_mn, idesc_o, 0u);     // dK = dS^T Q
-        mma_ts_x4<8, 128>(tdPT + 64, tST + 96, q_mn + 512, idesc_o, 1u);
-        mma_commit(bar_r2k);
+        if (leader) mma_ts_x4<8, 128>(tdPT, tST, do_mn, idesc_o, 0u);              // dV = P^T dO
+        if (leader) mma_ts_x4<8, 128>(tdPT, tST + 32, do_mn + 512, idesc_o, 1u);
+        if (leader) mma_ts_x4<8, 128>(tdPT + 64, tST + 64, q_mn, idesc_o, 0u);     // dK = dS^T Q
+        if (leader) mma_ts_x4<8, 128>(tdPT + 64, tST + 96, q_mn + 512, idesc_o, 1u);
+        if (leader) mma_commit(bar_r2k);
       }
     }
   } else if (warp < 8) {
@@ -442,14 +446,14 @@ win_tc_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         float nl0 = -CUDART_INF_F;
         if (z_next > 0.f && m_next > -CUDART_INF_F) nl0 = -(m_next + log2f(z_next));   // (a row whose keys are all masked keeps P = 0)
         load_state(pair + pair_step, m_next, z_next);
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_load + 8 * stage, (it >> 1) & 1, &abort_flag, prm.status, BAR_BLOAD))) break;
+        if (!mbar_wait_warp(bar_load + 8 * stage, (it >> 1) & 1, &abort_flag, prm.status, BAR_BLOAD)) break;
         nlse_s[ph][row] = nl0;
         nd_s[ph][row] = neg_row_dot<T>(tiles + 4 * kTileBytes, tiles + 3 * kTileBytes, row, d);
         mbar_arrive_warp(bar_pub, lane);
       }
-      if (prm.bias && !__all_sync(0xffffffffu, mbar_wait(bar_bias, ph, &abort_flag, prm.status, BAR_BIAS))) break;
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_r1, ph, &abort_flag, prm.status, BAR_R1))) break;
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_pub, ph, &abort_flag, prm.status, BAR_PUB))) break;
+      if (prm.bias && !mbar_wait_warp(bar_bias, ph, &abort_flag, prm.status, BAR_BIAS)) break;
+      if (!mbar_wait_warp(bar_r1, ph, &abort_flag, prm.status, BAR_R1)) break;
+      if (!mbar_wait_warp(bar_pub, ph, &abort_flag, prm.status, BAR_PUB)) break;
       tc_fence_after();
       {
         const float nlse = nlse_s[ph][row], nd = nd_s[ph][row];
@@ -502,7 +506,7 @@ win_tc_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       }
       tc_fence_before();
       mbar_arrive_warp(bar_phq, lane);
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_r2q, ph, &abort_flag, prm.status, BAR_R2Q))) break;
+      if (!mbar_wait_warp(bar_r2q, ph, &abort_flag, prm.status, BAR_R2Q)) break;
       tc_fence_after();
       T* dst = row_ok ? static_cast<T*>(prm.dq) + static_cast<int64_t>(b) * prm.dqs.b + hi * prm.dqs.h + static_cast<int64_t>(ri) * prm.dqs.r + 32 * half : nullptr;
       store_acc_half<T>(tdP + lane_off + 32 * half, dst, d - 32 * half, prm.scale);
@@ -510,7 +514,7 @@ win_tc_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       mbar_arrive_warp(bar_epi, lane);
       // the key side has consumed this pair's -LSE / -D (and the barrier phase that published them) before the next
       // pair's are published
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_r2k, ph, &abort_flag, prm.status, BAR_R2K))) break;
+      if (!mbar_wait_warp(bar_r2k, ph, &abort_flag, prm.status, BAR_R2K)) break;
     }
   } else {
     // ---------------- key-side warps: thread = (key row, half of the queries) ----------------
@@ -534,10 +538,10 @@ win_tc_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         if (bias_per_batch) stage_bias(sb, prm.bias, prm.bsb, prm.bsh, prm.bsq, prm.bsk, 2 * pair, 2, prm.batch, hi, N, warp & 7, 8, lane);
         else if (it == 0) stage_bias(sb, prm.bias, 0, prm.bsh, prm.bsq, prm.bsk, 0, 1, prm.batch, hi, N, warp & 7, 8, lane);
         mbar_arrive_warp(bar_bias, lane);
-        if (!__all_sync(0xffffffffu, mbar_wait(bar_bias, ph, &abort_flag, prm.status, BAR_BIAS))) break;   // all eight warps' rows
+        if (!mbar_wait_warp(bar_bias, ph, &abort_flag, prm.status, BAR_BIAS)) break;   // all eight warps' rows
       }
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_pub, ph, &abort_flag, prm.status, BAR_PUB))) break;   // -LSE, -D of the 128 queries
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_r1k, ph, &abort_flag, prm.status, BAR_R1K))) break;
+      if (!mbar_wait_warp(bar_pub, ph, &abort_flag, prm.status, BAR_PUB)) break;   // -LSE, -D of the 128 queries
+      if (!mbar_wait_warp(bar_r1k, ph, &abort_flag, prm.status, BAR_R1K)) break;
       tc_fence_after();
       {
         // this thread's 32 queries of the key's own sequence
@@ -610,7 +614,7 @@ win_tc_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       }
       tc_fence_before();
       mbar_arrive_warp(bar_phk, lane);
-      if (!__all_sync(0xffffffffu, mbar_wait(bar_r2k, ph, &abort_flag, prm.status, BAR_R2K))) break;
+      if (!mbar_wait_warp(bar_r2k, ph, &abort_flag, prm.status, BAR_R2K)) break;
       tc_fence_after();
       T* dvp = row_ok ? static_cast<T*>(prm.dv) + static_cast<int64_t>(b) * prm.dvs.b + hi * prm.dvs.h + static_cast<int64_t>(ri) * prm.dvs.r + 32 * half : nullptr;
       T* dkp = row_ok ? static_cast<T*>(prm.dk) + static_cast<int64_t>(b) * prm.dks.b + hi * prm.dks.h + static_cast<int64_t>(ri) * prm.dks.r + 32 * half : nullptr;
