@@ -584,7 +584,11 @@ extern "C" int64_t elsa_backward_workspace_bytes(int dtype, int batch, int heads
                                                  int has_bias, int is_causal, unsigned flags) {
   (void)is_causal;
   if (!dtype_ok(dtype) || batch < 1 || heads < 1 || n_ctx < 0 || head_dim < 1 || head_dim > 128) return -1;
-  if (tc_backward_ok(dtype, head_dim, n_ctx, batch * heads, has_bias != 0, flags)) return bwd_tc_workspace_bytes(batch * heads, n_ctx);
+  if (tc_backward_ok(dtype, head_dim, n_ctx, batch * heads, has_bias != 0, flags)) {
+    // (a biased problem runs there only when dbias is asked for, else on the wide-head kernels: room for either)
+    const int64_t tc = bwd_tc_workspace_bytes(batch * heads, n_ctx);
+    return has_bias ? std::max(tc, bwd_tcw_workspace_bytes(batch * heads, n_ctx)) : tc;
+  }
   // (the fp32 tensor-core route is not taken when dbias is asked for: the larger of the two needs covers both)
   if (tc3_backward_ok(dtype, head_dim, n_ctx, batch * heads, has_bias != 0, flags))
     return std::max(bwd_tc3_workspace_bytes(batch * heads, n_ctx, n_ctx), 2 * bwd_state_bytes(batch, heads, n_ctx));
@@ -614,7 +618,10 @@ static int backward_impl(const void* q, const void* k, const void* v, const void
   char* ws = static_cast<char*>(workspace);
   float* row_d = reinterpret_cast<float*>(ws);
   float* row_lse = reinterpret_cast<float*>(ws + bwd_state_bytes(batch, heads, n_ctx));
-  const bool use_tc = dbias == nullptr && tc_backward_ok(dtype, head_dim, n_ctx, batch * heads, bias != nullptr, flags);
+  // d <= 64, 16-bit: the five-contraction kernel, for a biased problem only when its gradient is asked for.  It reads the bias
+  // and writes dbias once, where the two kernels of bwd_tcw.cu read the bias twice, but adds dQ in arrival order; without a
+  // bias gradient the biased backward keeps the order-independent kernels (its dq repeats bit for bit).
+  const bool use_tc = (bias == nullptr) == (dbias == nullptr) && tc_backward_ok(dtype, head_dim, n_ctx, batch * heads, bias != nullptr, flags);
   const bool use_tc3 = (dbias == nullptr || bias != nullptr) && tc3_backward_ok(dtype, head_dim, n_ctx, batch * heads, bias != nullptr, flags);
   // (the wide-head kernels also take biased problems, with or without a bias gradient)
   const bool use_tcw = !use_tc && !use_tc3 && (dbias == nullptr || bias != nullptr) &&

@@ -1,6 +1,6 @@
 // Backward on the 5th-generation tensor cores: exact recompute from the saved row statistics,
 // fp16 / bf16 inputs, head dim 64 (or a smaller multiple of 8, zero-padded to 64 columns by the TMA box), causal or
-// not, no bias.  Five contractions per (key tile, query
+// not, with or without an additive bias and its gradient.  Five contractions per (key tile, query
 // tile) pair -- the algorithmic minimum -- all as tcgen05.mma with TMEM accumulators:
 //
 //   S^T  = K Q^T          [128 keys x 128 queries]   TMEM (K) x smem (Q, K-major)          N = 128
@@ -77,6 +77,9 @@ struct BwdTcParams {
   int n_keys, key_offset;                      // K/V rows of this launch and the sequence index of the first one
   int head_dim;                                // real columns of q, k, v, dout and the gradients (<= 64)
   float scale, scale_log2;
+  const float* bias; int64_t bsb, bsh, bsq, bsk;   // additive bias [.., N, N] (natural-log units); BIAS instantiation only
+  float* dbias; int64_t dsb, dsh, dsq, dsk;        // its gradient or null; dbias_atomic: an axis is summed over CTAs
+  int dbias_atomic;
   int* status;   // the device's status word (mapped host memory)
 };
 
@@ -86,7 +89,7 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint
 }
 
 
-template <typename T>
+template <typename T, bool BIAS>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
               const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -337,9 +340,32 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       mbar_arrive(bar_kvt);
     }
 
+    // Bias: a warp's 32 lanes are 32 consecutive keys, so one query's bias values (and its gradient's) are one
+    // 128-byte line per load (store) of the warp.
+    const int key_c = min(key, NK - 1);
+    const float* bias_key = BIAS ? prm.bias + bi * prm.bsb + hi * prm.bsh + static_cast<int64_t>(key_c) * prm.bsk : nullptr;
+    float* dbias_key = BIAS && prm.dbias ? prm.dbias + bi * prm.dsb + hi * prm.dsh + static_cast<int64_t>(key_c) * prm.dsk : nullptr;
     for (int it = 0; alive && it < n_it; ++it) {
       const int st = it % kQStages;
       const int q_tile0 = (it_begin + it) * 128;
+      float bv[BIAS ? 64 : 1];
+      if constexpr (BIAS) {
+        // the 64 bias values of this thread, all in flight before the scores are looked at (rows beyond N: the last one's)
+        const int qf = q_tile0 + half * 64;
+        if (q_tile0 + 128 <= N) {
+          const float* bp = bias_key + static_cast<int64_t>(qf) * prm.bsq;
+#pragma unroll
+          for (int i = 0; i < 64; ++i) bv[i] = __ldg(bp + i * prm.bsq);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) bv[i] = __ldg(bias_key + static_cast<int64_t>(min(qf + i, N - 1)) * prm.bsq);
+        }
+        // the next tile's lines (two queries per lane, the warp's 32 keys) towards L2
+        const int qn = qf + 128 + lane;
+        const float* np = prm.bias + bi * prm.bsb + hi * prm.bsh + static_cast<int64_t>(min(k0 + (row & ~31), NK - 1)) * prm.bsk;
+        if (qn < N) prefetch_l2(np + static_cast<int64_t>(qn) * prm.bsq);
+        if (qn + 32 < N) prefetch_l2(np + static_cast<int64_t>(qn + 32) * prm.bsq);
+      }
       if (!mbar_wait_warp(bar_s, it & 1, &abort_flag, prm.status, BAR_SP)) { alive = false; break; }
       // the row statistics of this stage were written by the bulk copies that complete on q_full: observe that
       // barrier directly (it completed before the MMAs behind bar_s were issued, so this never spins)
@@ -362,11 +388,20 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
 #pragma unroll
         for (int i = 0; i < 32; ++i) { p[i] = __uint_as_float(r0[i]); p[32 + i] = __uint_as_float(r1[i]); }
       }
+      if constexpr (BIAS) {
+        const float2 l2e = make_float2(1.4426950408889634f, 1.4426950408889634f);
+#pragma unroll
+        for (int i = 0; i < 64; i += 2) {
+          const float2 x = __ffma2_rn(make_float2(p[i], p[i + 1]), c2, __fmul2_rn(make_float2(bv[i], bv[i + 1]), l2e));
+          p[i] = x.x; p[i + 1] = x.y;
+        }
+      }
+      const float2 cs2 = BIAS ? make_float2(1.f, 1.f) : c2;
 #pragma unroll
       for (int g = 0; g < 16; ++g) {
         const float4 nl = nl4[g];                                   // -LSE of 4 queries (warp-wide broadcast read)
-        const float2 x0 = __ffma2_rn(make_float2(p[4 * g], p[4 * g + 1]), c2, make_float2(nl.x, nl.y));
-        const float2 x1 = __ffma2_rn(make_float2(p[4 * g + 2], p[4 * g + 3]), c2, make_float2(nl.z, nl.w));
+        const float2 x0 = __ffma2_rn(make_float2(p[4 * g], p[4 * g + 1]), cs2, make_float2(nl.x, nl.y));
+        const float2 x1 = __ffma2_rn(make_float2(p[4 * g + 2], p[4 * g + 3]), cs2, make_float2(nl.z, nl.w));
         p[4 * g] = fast_exp2(x0.x); p[4 * g + 1] = fast_exp2(x0.y);
         p[4 * g + 2] = fast_exp2(x1.x); p[4 * g + 3] = fast_exp2(x1.y);
         if (masked) {
@@ -387,6 +422,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         tmem_ld32(tdP(half) + lane_off + 32 * ch, rp);
         tmem_wait_ld();
         uint32_t pk[16], dsk[16];
+        float ds_f[BIAS ? 32 : 1];
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
           const float4 nd = nd4[ch * 8 + g];                        // -D of 4 queries
@@ -395,10 +431,30 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
           const float2 t0 = __fadd2_rn(make_float2(__uint_as_float(rp[4 * g]), __uint_as_float(rp[4 * g + 1])), make_float2(nd.x, nd.y));
           const float2 t1 = __fadd2_rn(make_float2(__uint_as_float(rp[4 * g + 2]), __uint_as_float(rp[4 * g + 3])), make_float2(nd.z, nd.w));
           const float2 d0 = __fmul2_rn(p0, t0), d1 = __fmul2_rn(p1, t1);
+          if constexpr (BIAS) {
+            ds_f[4 * g] = d0.x; ds_f[4 * g + 1] = d0.y; ds_f[4 * g + 2] = d1.x; ds_f[4 * g + 3] = d1.y;
+          }
           pk[2 * g] = pack2<T>(p0.x, p0.y);
           pk[2 * g + 1] = pack2<T>(p1.x, p1.y);
           dsk[2 * g] = pack2<T>(d0.x, d0.y);
           dsk[2 * g + 1] = pack2<T>(d1.x, d1.y);
+        }
+        if constexpr (BIAS) {
+          // dbias = dS, before its rounding.  The common case is free of branches per element.
+          const int qf = q_tile0 + half * 64 + 32 * ch;
+          if (dbias_key && key_ok) {
+            float* dp = dbias_key + static_cast<int64_t>(qf) * prm.dsq;
+            if (!prm.dbias_atomic && qf + 32 <= N) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) dp[i * prm.dsq] = ds_f[i];
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                if (qf + i >= N) continue;
+                if (prm.dbias_atomic) atomicAdd(dp + i * prm.dsq, ds_f[i]); else dp[i * prm.dsq] = ds_f[i];
+              }
+            }
+          }
         }
         // the 32 dP^T columns of this chunk are in registers: P^T goes over their first 16, dS^T over the other 16
         tmem_st16(tdP(half) + lane_off + 32 * ch, pk);
@@ -528,7 +584,10 @@ dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq, int n_ctx, 
 
 }  // namespace
 
-bool bwd_tc_supported(int dtype, int head_dim, bool has_bias) { return fold_tc_supported(dtype, head_dim, has_bias); }
+bool bwd_tc_supported(int dtype, int head_dim, bool has_bias) {
+  (void)has_bias;
+  return fold_tc_supported(dtype, head_dim, false);
+}
 
 int64_t bwd_tc_workspace_bytes(int bh, int n_ctx) {
   const int64_t n_pad = align_up(n_ctx, 128);
@@ -571,11 +630,14 @@ static int bwd_tc_t(const BwdParams& p, const void* out, Strides os, const float
   prm.dks = p.dks; prm.dvs = p.dvs;
   prm.n_keys = NK; prm.key_offset = p.key_offset; prm.head_dim = p.head_dim;
   prm.scale = p.scale; prm.scale_log2 = p.scale_log2;
-  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(&bwd_tc_kernel<T>), kBwdSmem);
+  prm.bias = p.bias; prm.bsb = p.bsb; prm.bsh = p.bsh; prm.bsq = p.bsq; prm.bsk = p.bsk;
+  prm.dbias = p.dbias; prm.dsb = p.dsb; prm.dsh = p.dsh; prm.dsq = p.dsq; prm.dsk = p.dsk; prm.dbias_atomic = p.dbias_atomic;
+  const auto kernel = p.bias ? &bwd_tc_kernel<T, true> : &bwd_tc_kernel<T, false>;
+  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kBwdSmem);
   if (rc != ELSA_OK) return rc;
   if (NK > 0) {
     dim3 grid(static_cast<unsigned>((NK + 127) / 128), static_cast<unsigned>(bh));
-    bwd_tc_kernel<T><<<grid, kThreads, kBwdSmem, st>>>(mq, mk, mv, mdo, mdq, prm);
+    kernel<<<grid, kThreads, kBwdSmem, st>>>(mq, mk, mv, mdo, mdq, prm);
     ELSA_LAUNCH_CHECK();
   }
   if (p.dq_f32) {
@@ -590,7 +652,7 @@ static int bwd_tc_t(const BwdParams& p, const void* out, Strides os, const float
 
 int bwd_tc(const BwdParams& p, const void* out, Strides os, const float* row_m, const float* row_z, void* workspace,
            int dtype, cudaStream_t st) {
-  if (!bwd_tc_supported(dtype, p.head_dim, p.bias != nullptr) || p.dbias) return ELSA_ERR_UNSUPPORTED;
+  if (!bwd_tc_supported(dtype, p.head_dim, p.bias != nullptr) || (p.dbias && !p.bias)) return ELSA_ERR_UNSUPPORTED;
   if (p.dq_f32 && p.head_dim != 64) return ELSA_ERR_UNSUPPORTED;   // the caller's fp32 dQ is the accumulator: 64-wide rows
   if (dtype == ELSA_F16) return bwd_tc_t<__half>(p, out, os, row_m, row_z, workspace, dtype, st);
   return bwd_tc_t<__nv_bfloat16>(p, out, os, row_m, row_z, workspace, dtype, st);
