@@ -55,7 +55,7 @@ enum BarId { BAR_ROW = 40, BAR_STAGE = 41, BAR_FULL = 42, BAR_FREE = 43, BAR_SDP
 
 struct Bwd3Params {
   const float* nlse_pad; const float* nd_pad;   // [BH][n_pad]: -LSE, -D; padding rows hold -inf / 0
-  const uint32_t* amax_q; const uint32_t* amax_do; const uint32_t* amax_k; const uint32_t* amax_v;   // the plane headers
+  const float* inv_q; const float* inv_do; const float* inv_k; const float* inv_v;   // 1 / plane scale, [BH][128-row tiles]
   float* dq; float* dk; float* dv;
   Strides dqs, dks, dvs;
   int n_ctx, n_pad, bh, heads, is_causal;
@@ -96,7 +96,7 @@ __device__ __forceinline__ void split_store16(const float* x, uint32_t tp0, uint
 }
 
 // The scaled quantities of the fp16-plane scheme (all factors are powers of two; 1 with bf16 planes), s_x being the
-// plane scale of tensor x:
+// plane scale of the tile of tensor x:
 //   S' = s_q s_k S, dP' = s_do s_v dP        arrive in TMEM; the fold divides the factors out
 //   P' = P * 2^kLog2Unit                     probabilities are at most 1 (the unit rides in the exponent)
 //   dS' = dS * r                             r = the power of two that puts the largest |dS| of this ROW of this tile
@@ -278,10 +278,12 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     const int qi = q0 + row;
     const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
     // plane scales (powers of two; see abs_max16): S arrives times s_q s_k, dP times s_do s_v, dS leaves times the row scale of the tile
-    const float s_q = plane_scale(*prm.amax_q), s_do = plane_scale(*prm.amax_do);
-    const float s_k = plane_scale(*prm.amax_k), s_v = plane_scale(*prm.amax_v);
-    const float c = prm.scale_log2 / (s_q * s_k);
-    const float idp = 1.f / (s_do * s_v);
+    const int tiles_k = (NK + kPlaneRows - 1) / kPlaneRows;
+    const int64_t qt = static_cast<int64_t>(bh) * ((N + kPlaneRows - 1) / kPlaneRows) + q0 / kPlaneRows;
+    const float c_q = prm.scale_log2 * prm.inv_q[qt], i_do = prm.inv_do[qt];
+    const float* inv_k = prm.inv_k + static_cast<int64_t>(bh) * tiles_k;
+    const float* inv_v = prm.inv_v + static_cast<int64_t>(bh) * tiles_k;
+    float ik_next = n_t > 0 ? inv_k[0] : 1.f, iv_next = n_t > 0 ? inv_v[0] : 1.f;
     const float nlse = prm.nlse_pad[static_cast<int64_t>(bh) * prm.n_pad + qi];   // q0 + 127 < n_pad
     const float nd = prm.nd_pad[static_cast<int64_t>(bh) * prm.n_pad + qi];
     float inv_r = 1.f;                         // 1 / (r s_k) of the tile whose dQ_j is in flight
@@ -307,6 +309,8 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     };
 
     for (int j = 0; alive && j < n_t; ++j) {
+      const float ik = ik_next, c = c_q * ik, idp = i_do * iv_next;
+      if (j + 1 < n_t) { ik_next = inv_k[j + 1]; iv_next = inv_v[j + 1]; }
       if (!mbar_wait_warp(bar_sdp, j & 1, &abort_flag, prm.status, BAR_SDP)) { alive = false; break; }
       tc_fence_after();
       float ds[32];
@@ -385,7 +389,7 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         tc_fence_after();
         take_dq();
       }
-      inv_r = 1.f / (r_scale * s_k);
+      inv_r = pow2_inv(r_scale) * ik;
       // the planes of dS: 16 keys (8 TMEM columns per plane) at a time
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) split_store16<64>(ds + 16 * ch, tDS + lane_off, 16 * cq + 8 * ch);
@@ -581,12 +585,14 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const bool cta_tail = k0 + 128 > NK;       // some key rows of this CTA do not exist
     // plane scales (powers of two; see abs_max16): S^T arrives times s_q s_k, dP^T times s_do s_v; P^T leaves times
     // 2^kLog2Unit (the unit rides in the exponent), dS^T times this key row's scale for the tile
-    const float s_q = plane_scale(*prm.amax_q), s_do = plane_scale(*prm.amax_do);
-    const float s_k = plane_scale(*prm.amax_k), s_v = plane_scale(*prm.amax_v);
-    const float c = prm.scale_log2 / (s_q * s_k);
+    const int tiles_q = (N + kPlaneRows - 1) / kPlaneRows;
+    const int64_t kt = static_cast<int64_t>(bh) * ((NK + kPlaneRows - 1) / kPlaneRows) + k0 / kPlaneRows;
     const float k2 = exp2f(-kLog2Unit);                 // dS = P' * (dP + nd) * k2
-    const float idp = k2 / (s_do * s_v);
-    const float inv_v = k2 / s_do;                      // dV_i' = 2^kLog2Unit s_do dV_i
+    const float c_k = prm.scale_log2 * prm.inv_k[kt], i_v = k2 * prm.inv_v[kt];
+    const float* inv_q = prm.inv_q + static_cast<int64_t>(bh) * tiles_q;
+    const float* inv_do = prm.inv_do + static_cast<int64_t>(bh) * tiles_q;
+    float iq_next = n_it > 0 ? inv_q[it_begin >> 1] : 1.f, ido_next = n_it > 0 ? inv_do[it_begin >> 1] : 1.f;   // (64-query tiles: two per scale)
+    float inv_v = 1.f;                                  // dV_i' = 2^kLog2Unit s_do dV_i, of the tile in flight
     float inv_r = 1.f;                                  // 1 / (r s_q) of the tile whose dK_i is in flight
     // bias[query, key] of this thread's key column; the query offset is added per element
     const float* bias_col = nullptr;
@@ -613,6 +619,8 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
     for (int it = 0; it < n_it; ++it) {
       const int q_tile0 = (it_begin + it) * 64;
+      const float iq = iq_next, ido = ido_next, c = c_k * iq, idp = i_v * ido;
+      if (it + 1 < n_it) { iq_next = inv_q[(it_begin + it + 1) >> 1]; ido_next = inv_do[(it_begin + it + 1) >> 1]; }
       if (!mbar_wait_warp(bar_sdp, it & 1, &abort_flag, prm.status, BAR_SDP)) { alive = false; break; }
       // the tile's row statistics were written by the bulk copies that complete on its first slot's barrier: observe
       // that barrier directly (it completed before the MMAs behind bar_sdp were issued, so this never spins)
@@ -677,7 +685,8 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         tc_fence_after();
         take_acc();
       }
-      inv_r = 1.f / (r_scale * s_q);
+      inv_r = pow2_inv(r_scale) * iq;
+      inv_v = k2 * ido;
       split_store16<32>(p, tP + lane_off, 8 * cq);
       split_store16<32>(ds, tDS + lane_off, 8 * cq);
       tmem_wait_st();
@@ -701,43 +710,6 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_before();
   __syncthreads();
   if (warp == kProducerWarp) tmem_dealloc(tmem_base, kTmemCols);
-}
-
-// -D = -sum_d out*dout, -LSE = -(m + log2(max(z, 1e-30))) into the padded layout; padding: -D = 0, -LSE = -inf
-__global__ void __launch_bounds__(256)
-bwd3_preprocess_kernel(const float* __restrict__ out, const float* __restrict__ dout, const float* __restrict__ row_m,
-                       const float* __restrict__ row_z, float* __restrict__ nd_pad, float* __restrict__ nlse_pad,
-                       int heads, int n_ctx, int n_pad, int head_dim, Strides os, Strides gs) {
-  // blockIdx.y = (batch*head); x covers the n_pad padded rows, 16 lanes (16 bytes each) per row
-  const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = static_cast<int>(gid >> 4);
-  const int lane = static_cast<int>(gid & 15);
-  const int64_t b = blockIdx.y;
-  const bool in_pad = r < n_pad;
-  const bool real = in_pad && r < n_ctx;
-  float part = 0.f;
-  if (real && lane * 4 < head_dim) {
-    const int bi = static_cast<int>(b) / heads, hi = static_cast<int>(b) - bi * heads;
-    const float4 o = *reinterpret_cast<const float4*>(out + bi * os.b + hi * os.h + static_cast<int64_t>(r) * os.r + lane * 4);
-    const float4 g = *reinterpret_cast<const float4*>(dout + bi * gs.b + hi * gs.h + static_cast<int64_t>(r) * gs.r + lane * 4);
-    part = (o.x * g.x + o.y * g.y) + (o.z * g.z + o.w * g.w);
-  }
-  part += __shfl_xor_sync(0xffffffffu, part, 8);
-  part += __shfl_xor_sync(0xffffffffu, part, 4);
-  part += __shfl_xor_sync(0xffffffffu, part, 2);
-  part += __shfl_xor_sync(0xffffffffu, part, 1);
-  if (in_pad && lane == 0) {
-    const int64_t prow = b * n_pad + r;
-    if (real) {
-      nd_pad[prow] = -part;
-      // (a row whose keys are all masked by the bias has m = -inf, z = 0: -LSE = -inf keeps its P at 0)
-      const float rm = row_m[b * n_ctx + r], rz = row_z[b * n_ctx + r];
-      nlse_pad[prow] = (rz > 0.f && rm > -CUDART_INF_F) ? -(rm + log2f(rz)) : -CUDART_INF_F;
-    } else {
-      nd_pad[prow] = 0.f;
-      nlse_pad[prow] = -CUDART_INF_F;
-    }
-  }
 }
 
 }  // namespace
@@ -766,31 +738,26 @@ int bwd_tc3(const BwdParams& p, const void* out, Strides os, const float* row_m,
   char* v3 = k3 + kb;
   int rc;
   {
-    const dim3 pgrid(static_cast<unsigned>(cdiv64(static_cast<int64_t>(n_pad) * 16, 256)), static_cast<unsigned>(bh));
-    bwd3_preprocess_kernel<<<pgrid, 256, 0, st>>>(static_cast<const float*>(out), static_cast<const float*>(p.dout), row_m,
-                                                  row_z, nd_pad, nlse_pad, p.heads, N, n_pad, p.head_dim, os, p.gs);
-    ELSA_LAUNCH_CHECK();
-  }
-  {
     const void* xs[4] = {p.q, p.dout, p.k, p.v};
     const Strides sts[4] = {p.qs, p.gs, p.ks, p.vs};
     void* pls[4] = {q3, do3, k3, v3};
     const int rws[4] = {N, N, NK, NK};
-    if ((rc = fold_tc3_split_many(4, xs, sts, pls, rws, batch, p.heads, p.head_dim, st)) != ELSA_OK) return rc;
+    const SplitStats stats{1, static_cast<const float*>(out), os, row_m, row_z, nd_pad, nlse_pad};
+    if ((rc = fold_tc3_split_many(4, xs, sts, pls, rws, batch, p.heads, p.head_dim, st, &stats)) != ELSA_OK) return rc;
   }
 
   // planes as [kPlanes, B*H, rows, 64] 16-bit tensors: the "head" coordinate is (batch*head), the "batch" coordinate the plane
   const Strides sq = contiguous_strides(bh, N, 64), sk = contiguous_strides(bh, NK, 64);
   CUtensorMap mq128, mdo128, mq64, mdo64, mk128, mv128;
-  if ((rc = make_tmap_rows64(&mq128, q3 + kPlaneHeader, kPlaneDtype, N, bh, kPlanes, sq, 128)) != ELSA_OK) return rc;
-  if ((rc = make_tmap_rows64(&mdo128, do3 + kPlaneHeader, kPlaneDtype, N, bh, kPlanes, sq, 128)) != ELSA_OK) return rc;
-  if ((rc = make_tmap_rows64(&mq64, q3 + kPlaneHeader, kPlaneDtype, N, bh, kPlanes, sq, 64)) != ELSA_OK) return rc;
-  if ((rc = make_tmap_rows64(&mdo64, do3 + kPlaneHeader, kPlaneDtype, N, bh, kPlanes, sq, 64)) != ELSA_OK) return rc;
+  if ((rc = make_tmap_rows64(&mq128, q3 + fold_tc3_header_bytes(bh, N), kPlaneDtype, N, bh, kPlanes, sq, 128)) != ELSA_OK) return rc;
+  if ((rc = make_tmap_rows64(&mdo128, do3 + fold_tc3_header_bytes(bh, N), kPlaneDtype, N, bh, kPlanes, sq, 128)) != ELSA_OK) return rc;
+  if ((rc = make_tmap_rows64(&mq64, q3 + fold_tc3_header_bytes(bh, N), kPlaneDtype, N, bh, kPlanes, sq, 64)) != ELSA_OK) return rc;
+  if ((rc = make_tmap_rows64(&mdo64, do3 + fold_tc3_header_bytes(bh, N), kPlaneDtype, N, bh, kPlanes, sq, 64)) != ELSA_OK) return rc;
   Bwd3Params prm;
   if ((rc = device_status_word(&prm.status, nullptr)) != ELSA_OK) return rc;
   prm.nlse_pad = nlse_pad; prm.nd_pad = nd_pad;
-  prm.amax_q = reinterpret_cast<const uint32_t*>(q3) + kAmaxFinal; prm.amax_do = reinterpret_cast<const uint32_t*>(do3) + kAmaxFinal;
-  prm.amax_k = reinterpret_cast<const uint32_t*>(k3) + kAmaxFinal; prm.amax_v = reinterpret_cast<const uint32_t*>(v3) + kAmaxFinal;
+  prm.inv_q = reinterpret_cast<const float*>(q3); prm.inv_do = reinterpret_cast<const float*>(do3);
+  prm.inv_k = reinterpret_cast<const float*>(k3); prm.inv_v = reinterpret_cast<const float*>(v3);
   prm.dq = static_cast<float*>(p.dq); prm.dk = static_cast<float*>(p.dk); prm.dv = static_cast<float*>(p.dv);
   prm.dqs = p.dqs; prm.dks = p.dks; prm.dvs = p.dvs;
   prm.n_ctx = N; prm.n_pad = n_pad; prm.bh = bh; prm.heads = p.heads; prm.is_causal = p.is_causal;
@@ -799,8 +766,8 @@ int bwd_tc3(const BwdParams& p, const void* out, Strides os, const float* row_m,
   prm.bias = p.bias; prm.bsb = p.bsb; prm.bsh = p.bsh; prm.bsq = p.bsq; prm.bsk = p.bsk;
   prm.dbias = p.dbias; prm.dsb = p.dsb; prm.dsh = p.dsh; prm.dsq = p.dsq; prm.dsk = p.dsk; prm.dbias_atomic = p.dbias_atomic;
   if (NK > 0) {
-    if ((rc = make_tmap_rows64(&mk128, k3 + kPlaneHeader, kPlaneDtype, NK, bh, kPlanes, sk, 128)) != ELSA_OK) return rc;
-    if ((rc = make_tmap_rows64(&mv128, v3 + kPlaneHeader, kPlaneDtype, NK, bh, kPlanes, sk, 128)) != ELSA_OK) return rc;
+    if ((rc = make_tmap_rows64(&mk128, k3 + fold_tc3_header_bytes(bh, NK), kPlaneDtype, NK, bh, kPlanes, sk, 128)) != ELSA_OK) return rc;
+    if ((rc = make_tmap_rows64(&mv128, v3 + fold_tc3_header_bytes(bh, NK), kPlaneDtype, NK, bh, kPlanes, sk, 128)) != ELSA_OK) return rc;
   } else {
     mk128 = mv128 = mq64;   // never dereferenced: no key tile is visited
   }

@@ -2,14 +2,14 @@
 // split into a few 16-bit planes and a product a*b is formed from the cross terms of the planes, each an exact
 // 16-bit x 16-bit product accumulated in fp32 by tcgen05.mma (kind::f16).  Two forms, chosen at compile time
 // (ELSA_FP32_PLANES, tc_common.cuh):
-//   2 planes (default): x * 2^e = h0 + h1 in fp16 (11 + 11 significant bits; e puts the tensor's largest magnitude in
-//     [2^13, 2^14)), a*b = h0 h0 + h0 h1 + h1 h0 (dropped: h1 h1 <= 2^-22 relative).  This is the accuracy class of
+//   2 planes (default): x * 2^e = h0 + h1 in fp16 (11 + 11 significant bits; e puts the largest magnitude of a 128-row
+//     tile in [2^13, 2^14)), a*b = h0 h0 + h0 h1 + h1 h0 (dropped: h1 h1 <= 2^-22 relative).  This is the accuracy class of
 //     the reference's own fp32 route, 3xTF32 (src/elsa_twopass_clean/attention.py:280-282, 10 + 11 bits per operand),
 //     at half its tensor-pipe cost: a tf32 instruction covers half the K extent of an fp16 one.
 //   3 planes: x = b0 + b1 + b2 in bf16 (8 + 8 + 8 bits, no scaling needed), six cross terms of weight >= 2^-16
 //     (dropped: <= 2^-24 relative).  Twice the instructions; 2-3 x closer to fp64 on the forward.
 //
-// A pre-pass (absmax_kernel + split_planes_kernel) writes the planes of q, k, v once per forward call.  One CTA (576
+// A pre-pass (split_planes_kernel) writes the planes of q, k, v once per forward call.  One CTA (576
 // threads, 1 per SM) owns ONE 128-row query tile of one (batch*head) and one K partition, walked in 128-key tiles:
 //
 //   warp 16     TMA producer   the planes of the Q tile once; then 16 KB plane tiles through an 8-slot ring in the
@@ -25,9 +25,10 @@
 //                              output lives in registers (16 columns per thread) and takes in O_{j-1} with ordinary
 //                              fp32 additions
 //
-// Scales.  The plane scales of q, k, v are powers of two, so they come out exactly: the scores arrive times s_q s_k
-// (divided out together with the softmax scale), P is produced times 2^14 by adding 14 to the exponent of the
-// exponential (so the row sum and the output carry 2^14, the output also s_v), and the epilogue takes all of it out.
+// Scales.  The plane scales of the q, k, v tiles are powers of two, so they come out exactly: the scores of a tile pair
+// arrive times s_q s_k (divided out together with the softmax scale), O of a key tile times s_v (divided out when it is
+// taken into the running sum), and P is produced times 2^14 by adding 14 to the exponent of the exponential (so the row
+// sum and the output carry 2^14 until the epilogue).
 // With fp16 planes a weight must not exceed 1, so the reference max follows every key tile (no lazy rescale).
 //
 // The per-element work of the fold is about a dozen instructions; with one thread per row (four warps, one per
@@ -72,7 +73,7 @@ struct Fold3Params {
   int n_ctx, q_start, q_len, part_width, n_parts, bh, is_causal, summary_dtype;
   int n_keys, key_offset, head_dim;
   float scale_log2;
-  const uint32_t* amax_q; const uint32_t* amax_k; const uint32_t* amax_v;   // the plane headers
+  const float* inv_q; const float* inv_k; const float* inv_v;   // 1 / plane scale, [BH][128-row tiles]
   const float* bias; int64_t bsb, bsh, bsq, bsk;   // additive bias [.., N, N] (natural-log units) or null
   int heads;
   int* status;
@@ -106,81 +107,89 @@ __device__ __forceinline__ void store_row16(TS* dst, const float (&v)[16], int n
 
 // ---- the plane pre-pass: up to four tensors per launch (blockIdx.z selects the tensor) ----
 struct SplitJobs {
-  const float* x[4]; Strides st[4]; uint32_t* header[4]; int rows[4];
+  const float* x[4]; Strides st[4]; float* inv_scale[4]; uint16_t* planes[4]; int rows[4];
+  // statistics of the backward, computed with the tensor of job `stat_job` (dout) while it is in registers:
+  // -D = -sum_d out*dout and -LSE = -(m + log2 z), padded to whole tiles with 0 and -inf (stat_job < 0: none)
+  int stat_job;
+  const float* out; Strides os; const float* row_m; const float* row_z; float* nd_pad; float* nlse_pad;
 };
 
-// largest |x| of each [B, H, rows, cols] fp32 view: kAmaxBlocks blocks per tensor stride over its rows and write one
-// partial maximum each into the tensor's plane header (bit patterns: non-negative floats order like integers); no
-// atomics, nothing to zero beforehand
-__global__ void __launch_bounds__(256)
-absmax_kernel(const __grid_constant__ SplitJobs jobs, int heads, int bh, int cols) {
-  __shared__ float wmax[8];
-  const int job = blockIdx.z;
-  const float* x = jobs.x[job];
-  const Strides st = jobs.st[job];
-  const int rows = jobs.rows[job];
-  const int c = static_cast<int>(threadIdx.x & 15) * 4;          // 16 threads per row of 64
-  float m = 0.f;
-  if (c < cols) {
-    const int64_t total = static_cast<int64_t>(bh) * rows;
-    for (int64_t fr = blockIdx.x * 16 + static_cast<int>(threadIdx.x >> 4); fr < total; fr += gridDim.x * 16) {
-      const int g = static_cast<int>(fr / rows), r = static_cast<int>(fr - static_cast<int64_t>(g) * rows);
-      const int b = g / heads, h = g - b * heads;
-      const float4 v = *reinterpret_cast<const float4*>(x + b * st.b + h * st.h + static_cast<int64_t>(r) * st.r + c);
-      m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int w = 1; w < 8; ++w) m = fmaxf(m, wmax[w]);
-    jobs.header[job][blockIdx.x] = (m > 0.f && m <= 3.0e38f) ? __float_as_uint(m) : 0u;
-  }
-}
-
-// x (4 consecutive fp32 of a row of `cols` values, any strides) times the tensor's plane scale -> kPlanes 16-bit
-// planes [kPlanes][B*H][rows][64] behind the header, contiguous; columns beyond `cols` are written as zeros (a head dim
-// below 64 becomes a zero-padded 64-column operand).  The tensor's largest magnitude is the maximum of the partial
-// maxima in its header; block (0, 0) also leaves it in header[kAmaxFinal] for the kernels that undo the scale.
+// One block per 128-row tile of one (batch*head): [128, cols] fp32 (any strides) times the tile's plane scale ->
+// kPlanes 16-bit planes [kPlanes][B*H][rows][64], contiguous; columns beyond `cols` are written as zeros (a head dim
+// below 64 becomes a zero-padded 64-column operand), 1 / scale goes to inv_scale[bh][tile].
+// Bound: HBM, one read of the tensor and one write of as many bytes.  The tile is kept in registers between the search
+// for its largest magnitude and the split.  One scale per tensor instead needs the maximum of all of it first: a pass of
+// its own over the tensor (21 us of 616 per fwd+bwd at (1,8,4096,64), twice; 5.2 of 30.7 us of a forward at 1024).
 __global__ void __launch_bounds__(256)
 split_planes_kernel(const __grid_constant__ SplitJobs jobs, int heads, int bh, int cols) {
-  __shared__ uint32_t amax_s;
+  __shared__ float wmax[8];
   const int job = blockIdx.z;
   const int rows = jobs.rows[job];
-  uint32_t* header = jobs.header[job];
-  if (kPlanes == 2) {
-    if (threadIdx.x < 32) {
-      uint32_t m = max(header[threadIdx.x], header[threadIdx.x + 32]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if (threadIdx.x == 0) {
-        amax_s = m;
-        if (blockIdx.x == 0 && blockIdx.y == 0) header[kAmaxFinal] = m;
-      }
-    }
-    __syncthreads();
-  } else if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) {
-    header[kAmaxFinal] = 0u;
-  }
-  const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;    // 16 threads per row of 64
-  const int r = static_cast<int>(idx >> 4), c = static_cast<int>(idx & 15) * 4;
-  if (r >= rows) return;
+  const int r0 = blockIdx.x * kPlaneRows;
+  if (r0 >= rows) return;
   const int g = blockIdx.y, b = g / heads, h = g - b * heads;
   const Strides st = jobs.st[job];
-  const float sc = kPlanes == 2 ? plane_scale(amax_s) : 1.f;
-  const float4 v = c < cols ? *reinterpret_cast<const float4*>(jobs.x[job] + b * st.b + h * st.h + static_cast<int64_t>(r) * st.r + c)
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
-  uint32_t w0[kPlanes], w1[kPlanes];
-  split_planes_pair(v.x * sc, v.y * sc, w0);
-  split_planes_pair(v.z * sc, v.w * sc, w1);
-  uint16_t* planes = reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(header) + kPlaneHeader);
-  const int64_t plane_elems = static_cast<int64_t>(bh) * rows * 64;
-  const int64_t off = (static_cast<int64_t>(g) * rows + r) * 64 + c;
+  const int c = static_cast<int>(threadIdx.x & 15) * 4, rt = static_cast<int>(threadIdx.x >> 4);   // 16 threads per row of 64
+  const float* x = jobs.x[job] + b * st.b + h * st.h + c;
+  float4 v[8];
 #pragma unroll
-  for (int p = 0; p < kPlanes; ++p) *reinterpret_cast<uint2*>(planes + p * plane_elems + off) = make_uint2(w0[p], w1[p]);
+  for (int i = 0; i < 8; ++i) {
+    const int r = r0 + rt + 16 * i;
+    v[i] = (c < cols && r < rows) ? *reinterpret_cast<const float4*>(x + static_cast<int64_t>(r) * st.r) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (job == jobs.stat_job) {
+    const float* o = jobs.out + b * jobs.os.b + h * jobs.os.h + c;
+    const int n_pad = (rows + kPlaneRows - 1) / kPlaneRows * kPlaneRows;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = r0 + rt + 16 * i;
+      float part = 0.f;
+      if (c < cols && r < rows) {
+        const float4 ov = *reinterpret_cast<const float4*>(o + static_cast<int64_t>(r) * jobs.os.r);
+        part = (ov.x * v[i].x + ov.y * v[i].y) + (ov.z * v[i].z + ov.w * v[i].w);
+      }
+#pragma unroll
+      for (int sft = 8; sft > 0; sft >>= 1) part += __shfl_xor_sync(0xffffffffu, part, sft);
+      if ((threadIdx.x & 15) == 0) {
+        float nd = 0.f, nlse = -CUDART_INF_F;
+        if (r < rows) {
+          nd = -part;
+          // (a row whose keys are all masked by the bias has m = -inf, z = 0: -LSE = -inf keeps its P at 0)
+          const float rm = jobs.row_m[static_cast<int64_t>(g) * rows + r], rz = jobs.row_z[static_cast<int64_t>(g) * rows + r];
+          if (rz > 0.f && rm > -CUDART_INF_F) nlse = -(rm + log2f(rz));
+        }
+        jobs.nd_pad[static_cast<int64_t>(g) * n_pad + r] = nd;
+        jobs.nlse_pad[static_cast<int64_t>(g) * n_pad + r] = nlse;
+      }
+    }
+  }
+  float sc = 1.f;
+  if (kPlanes == 2) {
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = fmaxf(m, wmax[w]);
+    sc = plane_scale((m > 0.f && m <= 3.0e38f) ? __float_as_uint(m) : 0u);
+  }
+  if (threadIdx.x == 0) jobs.inv_scale[job][static_cast<int64_t>(g) * ((rows + kPlaneRows - 1) / kPlaneRows) + blockIdx.x] = pow2_inv(sc);
+  uint16_t* planes = jobs.planes[job];
+  const int64_t plane_elems = static_cast<int64_t>(bh) * rows * 64;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = r0 + rt + 16 * i;
+    if (r >= rows) break;
+    uint32_t w0[kPlanes], w1[kPlanes];
+    split_planes_pair(v[i].x * sc, v[i].y * sc, w0);
+    split_planes_pair(v[i].z * sc, v[i].w * sc, w1);
+    const int64_t off = (static_cast<int64_t>(g) * rows + r) * 64 + c;
+#pragma unroll
+    for (int p = 0; p < kPlanes; ++p) *reinterpret_cast<uint2*>(planes + p * plane_elems + off) = make_uint2(w0[p], w1[p]);
+  }
 }
 
 template <bool BIAS>
@@ -330,10 +339,13 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const int row = qd * 32 + lane;                         // row within the tile == TMEM lane
     const int qi = q0 + row;
     const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
-    // the scores arrive multiplied by the plane scales of q and k (powers of two): taken out with the softmax scale
-    const float c = prm.scale_log2 / (plane_scale(*prm.amax_q) * plane_scale(*prm.amax_k));
-    // with a bias the scores are moved to the log2 domain at once (s c + b log2 e) and the scale below becomes 1
-    const float cc = BIAS ? 1.f : c;
+    // the scores of a tile pair arrive multiplied by the plane scales of its q and k tiles (powers of two): taken out
+    // with the softmax scale
+    const int tiles_k = (prm.n_keys + kPlaneRows - 1) / kPlaneRows;
+    const float cq_scale = prm.scale_log2 * prm.inv_q[static_cast<int64_t>(bh) * ((prm.n_ctx + kPlaneRows - 1) / kPlaneRows) + min(q0, prm.n_ctx - 1) / kPlaneRows];
+    const float* inv_k = prm.inv_k + static_cast<int64_t>(bh) * tiles_k + k_begin / kPlaneRows;
+    const float* inv_v = prm.inv_v + static_cast<int64_t>(bh) * tiles_k + k_begin / kPlaneRows;
+    float ik_next = n_t > 0 ? inv_k[0] : 1.f, iv_next = n_t > 0 ? inv_v[0] : 1.f, iv = 1.f;   // iv: of the tile whose O is in flight
     const float* bias_row = nullptr;
     if constexpr (BIAS) {
       const int bi = bh / prm.heads, hi = bh - bi * prm.heads;
@@ -351,10 +363,14 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       tmem_ld16(tO + lane_off + 16 * cq, r);
       tmem_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 16; ++i) o_run[i] += __uint_as_float(r[i]);
+      for (int i = 0; i < 16; ++i) o_run[i] = fmaf(__uint_as_float(r[i]), iv, o_run[i]);
     };
 
     for (int j = 0; j < n_t; ++j) {
+      const float c = cq_scale * ik_next, iv_this = iv_next;
+      if (j + 1 < n_t) { ik_next = inv_k[j + 1]; iv_next = inv_v[j + 1]; }
+      // with a bias the scores are moved to the log2 domain at once (s c + b log2 e) and the scale below becomes 1
+      const float cc = BIAS ? 1.f : c;
       if (!mbar_wait_warp(bar_s, j & 1, &abort_flag, prm.status, BAR_S)) { alive = false; break; }
       tc_fence_after();
       float sv[32];
@@ -437,6 +453,7 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         tc_fence_after();
         take_o();
       }
+      iv = iv_this;
       if (move) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) o_run[i] *= alpha;
@@ -476,13 +493,12 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       if (alive) {
         const float ztot = (row_sum[0][row] + row_sum[1][row]) + (row_sum[2][row] + row_sum[3][row]);
-        // zsum carries kPlaneUnit, o_run kPlaneUnit and the plane scale of v (powers of two: taken out exactly)
+        // zsum and o_run carry kPlaneUnit (a power of two: taken out exactly)
         const float f = (m_true == -CUDART_INF_F) ? 0.f : exp2f(m_ref - m_true - kLog2Unit);
-        const float fo = f / plane_scale(*prm.amax_v);
         z_out = ztot * f;
         m_out = z_out > 0.f ? m_true : -CUDART_INF_F;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) o_run[i] = z_out > 0.f ? o_run[i] * fo : 0.f;
+        for (int i = 0; i < 16; ++i) o_run[i] = z_out > 0.f ? o_run[i] * f : 0.f;
       }
     }
     if (row_ok && (alive || n_t == 0)) {
@@ -508,42 +524,46 @@ bool fold_tc3_supported(int dtype, int head_dim, bool has_bias) {
   return dtype == ELSA_F32 && head_dim >= 8 && head_dim <= 64 && head_dim % 8 == 0 && fold_tc_supported(ELSA_BF16, 64, false);
 }
 
-// a tensor's plane buffer: a header (kAmaxBlocks partial maxima and the final one) + [kPlanes][bh][rows][64] 16-bit
+// a tensor's plane buffer: a header (1 / scale of every 128-row tile) + [kPlanes][bh][rows][64] 16-bit
+int64_t fold_tc3_header_bytes(int bh, int rows) { return align_up(static_cast<int64_t>(bh) * cdiv64(rows, kPlaneRows) * 4, 512); }
 int64_t fold_tc3_plane_bytes(int bh, int rows) {
-  return kPlaneHeader + align_up(static_cast<int64_t>(kPlanes) * bh * rows * 64 * 2, 256);
+  return fold_tc3_header_bytes(bh, rows) + align_up(static_cast<int64_t>(kPlanes) * bh * rows * 64 * 2, 256);
 }
 
 // the planes of up to four fp32 tensors ([B, H, rows[i], cols] views with strides st[i]) into planes[i]
-// (fold_tc3_plane_bytes each): two launches for all of them
+// (fold_tc3_plane_bytes each), one launch for all of them
 int fold_tc3_split_many(int n, const void* const* x, const Strides* st, void* const* planes, const int* rows, int batch,
-                        int heads, int cols, cudaStream_t stream) {
+                        int heads, int cols, cudaStream_t stream, const SplitStats* stats) {
   if (n < 1 || n > 4) return ELSA_ERR_INVALID_ARGUMENT;
   SplitJobs jobs;
   int n_jobs = 0, max_rows = 0;
+  const int bh = batch * heads;
+  jobs.stat_job = -1;
   for (int i = 0; i < n; ++i) {
     if (rows[i] <= 0) continue;
     if ((st[i].b | st[i].h | st[i].r) % 4 != 0 || (reinterpret_cast<uintptr_t>(x[i]) & 15u)) return ELSA_ERR_INVALID_ARGUMENT;
     jobs.x[n_jobs] = static_cast<const float*>(x[i]); jobs.st[n_jobs] = st[i];
-    jobs.header[n_jobs] = static_cast<uint32_t*>(planes[i]); jobs.rows[n_jobs] = rows[i];
+    jobs.inv_scale[n_jobs] = static_cast<float*>(planes[i]);
+    jobs.planes[n_jobs] = reinterpret_cast<uint16_t*>(static_cast<char*>(planes[i]) + fold_tc3_header_bytes(bh, rows[i]));
+    jobs.rows[n_jobs] = rows[i];
     max_rows = std::max(max_rows, rows[i]);
+    if (stats && stats->tensor == i) {
+      jobs.stat_job = n_jobs;
+      jobs.out = stats->out; jobs.os = stats->os; jobs.row_m = stats->row_m; jobs.row_z = stats->row_z;
+      jobs.nd_pad = stats->nd_pad; jobs.nlse_pad = stats->nlse_pad;
+    }
     ++n_jobs;
   }
   if (n_jobs == 0) return ELSA_OK;
-  for (int i = n_jobs; i < 4; ++i) { jobs.x[i] = jobs.x[0]; jobs.st[i] = jobs.st[0]; jobs.header[i] = jobs.header[0]; jobs.rows[i] = 0; }
-  const int bh = batch * heads;
-  if (kPlanes == 2) {
-    absmax_kernel<<<dim3(kAmaxBlocks, 1, static_cast<unsigned>(n_jobs)), 256, 0, stream>>>(jobs, heads, bh, cols);
-    ELSA_LAUNCH_CHECK();
-  }
-  const dim3 grid(static_cast<unsigned>(cdiv64(static_cast<int64_t>(max_rows) * 16, 256)), static_cast<unsigned>(bh),
-                  static_cast<unsigned>(n_jobs));
+  for (int i = n_jobs; i < 4; ++i) { jobs.x[i] = jobs.x[0]; jobs.st[i] = jobs.st[0]; jobs.inv_scale[i] = jobs.inv_scale[0]; jobs.planes[i] = jobs.planes[0]; jobs.rows[i] = 0; }
+  const dim3 grid(static_cast<unsigned>(cdiv64(max_rows, kPlaneRows)), static_cast<unsigned>(bh), static_cast<unsigned>(n_jobs));
   split_planes_kernel<<<grid, 256, 0, stream>>>(jobs, heads, bh, cols);
   ELSA_LAUNCH_CHECK();
   return ELSA_OK;
 }
 
 int fold_tc3_split(const void* x, Strides st, void* planes, int batch, int heads, int rows, int cols, cudaStream_t stream) {
-  return fold_tc3_split_many(1, &x, &st, &planes, &rows, batch, heads, cols, stream);
+  return fold_tc3_split_many(1, &x, &st, &planes, &rows, batch, heads, cols, stream, nullptr);
 }
 
 // p.q3 / p.k3 / p.v3: the plane buffers written by fold_tc3_split for the whole problem (all query rows / this
@@ -555,13 +575,12 @@ int fold_tc3(const FoldParams& p, cudaStream_t st) {
   int rc;
   // planes as a [kPlanes, B*H, rows, 64] 16-bit tensor: the "head" coordinate is (batch*head), the "batch" coordinate the plane
   const Strides sq = contiguous_strides(p.bh, p.n_ctx, 64), sk = contiguous_strides(p.bh, p.n_keys, 64);
-  if ((rc = make_tmap_rows64(&mq, static_cast<const char*>(p.q3) + kPlaneHeader, kPlaneDtype, p.n_ctx, p.bh, kPlanes, sq, 128)) != ELSA_OK) return rc;
-  if ((rc = make_tmap_rows64(&mk, static_cast<const char*>(p.k3) + kPlaneHeader, kPlaneDtype, p.n_keys, p.bh, kPlanes, sk, 128)) != ELSA_OK) return rc;
-  if ((rc = make_tmap_rows64(&mv, static_cast<const char*>(p.v3) + kPlaneHeader, kPlaneDtype, p.n_keys, p.bh, kPlanes, sk, 128)) != ELSA_OK) return rc;
+  if ((rc = make_tmap_rows64(&mq, static_cast<const char*>(p.q3) + fold_tc3_header_bytes(p.bh, p.n_ctx), kPlaneDtype, p.n_ctx, p.bh, kPlanes, sq, 128)) != ELSA_OK) return rc;
+  if ((rc = make_tmap_rows64(&mk, static_cast<const char*>(p.k3) + fold_tc3_header_bytes(p.bh, p.n_keys), kPlaneDtype, p.n_keys, p.bh, kPlanes, sk, 128)) != ELSA_OK) return rc;
+  if ((rc = make_tmap_rows64(&mv, static_cast<const char*>(p.v3) + fold_tc3_header_bytes(p.bh, p.n_keys), kPlaneDtype, p.n_keys, p.bh, kPlanes, sk, 128)) != ELSA_OK) return rc;
   Fold3Params prm;
   prm.m = p.m; prm.z = p.z; prm.s = p.s;
-  prm.amax_q = static_cast<const uint32_t*>(p.q3) + kAmaxFinal; prm.amax_k = static_cast<const uint32_t*>(p.k3) + kAmaxFinal;
-  prm.amax_v = static_cast<const uint32_t*>(p.v3) + kAmaxFinal;
+  prm.inv_q = static_cast<const float*>(p.q3); prm.inv_k = static_cast<const float*>(p.k3); prm.inv_v = static_cast<const float*>(p.v3);
   if ((rc = device_status_word(&prm.status, nullptr)) != ELSA_OK) return rc;
   prm.n_ctx = p.n_ctx; prm.q_start = p.q_start; prm.q_len = p.q_len; prm.part_width = p.part_width;
   prm.n_parts = p.n_parts; prm.bh = p.bh; prm.is_causal = p.is_causal; prm.summary_dtype = p.summary_dtype;

@@ -317,22 +317,21 @@ __device__ __forceinline__ void st_global_v8(float* p, const float (&r)[8]) {
 // ELSA_FP32_PLANES == 3: x = a0 + a1 + a2 with three bf16 terms (8 + 8 + 8 significant bits, the full exponent range;
 //   six cross products of weight >= 2^-16 per contraction).
 // ELSA_FP32_PLANES == 2: x * 2^e = h0 + h1 with two fp16 terms (11 + 11 significant bits; three cross products
-//   h0 h0 + h0 h1 + h1 h0 per contraction, the accuracy class of 3xTF32).  fp16 has five exponent bits, so every tensor
-//   is multiplied by a power of two that puts its largest magnitude in [2^13, 2^14): elements down to 2^-16 of the
-//   largest keep all 22 bits, smaller ones lose low bits gradually (absolute error below 2^-38 of the largest).
+//   h0 h0 + h0 h1 + h1 h0 per contraction, the accuracy class of 3xTF32).  fp16 has five exponent bits, so every
+//   128-row tile is multiplied by a power of two that puts its largest magnitude in [2^13, 2^14): elements down to 2^-16
+//   of the tile's largest keep all 22 bits, smaller ones lose low bits gradually (absolute error below 2^-38 of the largest).
 #ifndef ELSA_FP32_PLANES
 #define ELSA_FP32_PLANES 2
 #endif
 constexpr int kPlanes = ELSA_FP32_PLANES;
 static_assert(kPlanes == 2 || kPlanes == 3, "fp32 operands are split into two fp16 or three bf16 planes");
 constexpr float kLog2Unit = kPlanes == 2 ? 14.f : 0.f;        // log2 of what a probability (<= 1) is multiplied by before its split
-constexpr int kAmaxBlocks = 64, kAmaxFinal = 64;               // header words: partial |x| maxima (bit patterns), then the final one
-constexpr int kPlaneHeader = 512;                              // bytes in front of a tensor's planes
+constexpr int kPlaneRows = 128;                                // rows that share one scale
 constexpr uint32_t kPlaneFmt = kPlanes == 3 ? 1u : 0u;         // tcgen05 operand format: bf16 / fp16
 constexpr int kPlaneDtype = kPlanes == 3 ? ELSA_BF16 : ELSA_F16;
 
-// the power of two that scales a tensor whose largest magnitude has the bit pattern `absmax_bits` (0 for an all-zero
-// tensor) into [2^13, 2^14); 1 for bf16 planes
+// the power of two that scales values whose largest magnitude has the bit pattern `absmax_bits` (0 when all are zero)
+// into [2^13, 2^14); 1 for bf16 planes
 __device__ __forceinline__ float plane_scale(uint32_t absmax_bits) {
   if (kPlanes == 3) return 1.f;
   int e = static_cast<int>(absmax_bits >> 23) - 127;         // floor(log2(absmax)) for a normal number
@@ -340,6 +339,9 @@ __device__ __forceinline__ float plane_scale(uint32_t absmax_bits) {
   e = max(-100, min(100, e));
   return __uint_as_float(static_cast<uint32_t>(127 + 13 - e) << 23);
 }
+
+// 1 / x of a power of two in the normal range, exactly and without a division
+__device__ __forceinline__ float pow2_inv(float x) { return __uint_as_float(0x7F000000u - __float_as_uint(x)); }
 
 // a pair of values -> its kPlanes packed 16-bit pairs (element 0 in the low half), leading plane first: round to
 // nearest each time, remainders exact
