@@ -34,6 +34,9 @@
 //   warp 12     TMA producer: K, V once; Q_i, dO_i, -LSE_i, -D_i into a 2-stage ring
 //   warp 13     MMA issuer
 //   (register budget re-balanced with setmaxnreg: 168 / 168 / 96 / 80 per thread = 4 x 128, the launch allocation)
+// Every mbarrier that warps feed counts one arrival per warp: with one per thread the arrivals alone were 640 of the
+// 1440 shared-memory wavefronts of a tile pair (fwd+bwd at (8,3,4097,64) fp16 562 -> 552 us, causal bf16 (1,8,16384,64)
+// 1288 -> 1264 us).
 //
 // TMEM columns: S^T [0,128) dP^T [128,256) dV [256,320) dK [320,384) dQ [384,448) K [448,480) V [480,512).
 // Within the 64 dP^T columns of a half, chunk ch keeps P^T in [32 ch, +16) and dS^T in [32 ch + 16, +16).
@@ -137,11 +140,11 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
     abort_flag = 0;
     mbar_init(bar_kv, 1);
     for (int st = 0; st < kQStages; ++st) { mbar_init(bar_q_full(st), 1); mbar_init(bar_q_free(st), 1); }
-    mbar_init(bar_s, 1); mbar_init(bar_dpx(0), 1); mbar_init(bar_dpx(1), 1); mbar_init(bar_lds, 256);
-    mbar_init(bar_pds, 256);
-    mbar_init(bar_dq_free, 128);
+    mbar_init(bar_s, 1); mbar_init(bar_dpx(0), 1); mbar_init(bar_dpx(1), 1); mbar_init(bar_lds, 8);
+    mbar_init(bar_pds, 8);
+    mbar_init(bar_dq_free, 4);
     mbar_init(bar_done, 1);
-    mbar_init(bar_kvt, 256);
+    mbar_init(bar_kvt, 8);
     fence_mbar_init();
   }
   if (warp == 12) {
@@ -286,7 +289,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       tmem_ld32(tdQ + lane_off + 32, r1);
       tmem_wait_ld();
       tc_fence_before();
-      mbar_arrive(bar_dq_free);
+      mbar_arrive_warp(bar_dq_free, lane);
       // Stage the 128 x 64 fp32 tile in shared memory (two 32-column blocks, 128-byte swizzle) and let the TMA
       // unit add it into the global accumulator: whole 128-byte lines per reduction instead of one 16-byte
       // piece per lane, and no LSU traffic that would delay the MMA issue slots of this scheduler.
@@ -337,7 +340,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       tmem_st32((half == 0 ? tK : tV) + lane_off, w);
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(bar_kvt);
+      mbar_arrive_warp(bar_kvt, lane);
     }
 
     // Bias: a warp's 32 lanes are 32 consecutive keys, so one query's bias values (and its gradient's) are one
@@ -384,7 +387,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
         tmem_ld32(tS(half) + lane_off + 32, r1);
         tmem_wait_ld();
         tc_fence_before();
-        mbar_arrive(bar_lds);       // the S^T columns may be overwritten with the next query tile's scores
+        mbar_arrive_warp(bar_lds, lane);       // the S^T columns may be overwritten with the next query tile's scores
 #pragma unroll
         for (int i = 0; i < 32; ++i) { p[i] = __uint_as_float(r0[i]); p[32 + i] = __uint_as_float(r1[i]); }
       }
@@ -472,7 +475,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant_
       fence_proxy_async_smem();
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(bar_pds);
+      mbar_arrive_warp(bar_pds, lane);
     }
 
     // ---- epilogue: dK, dV of this key tile (tcgen05.ld is warp-collective: only the stores are predicated) ----
