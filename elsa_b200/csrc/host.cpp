@@ -257,7 +257,12 @@ struct AttentionBackward : public torch::autograd::Node {
     if (go.scalar_type() != q.scalar_type()) go = go.to(q.scalar_type());
     c10::cuda::CUDAGuard guard(q.device());
     at::Tensor dbias;
-    if (bias_grad) dbias = at::zeros_like(bias.t);
+    if (bias_grad) {
+      // Sums over a broadcast axis and pairs that the causal rule leaves out need zeros.  Otherwise the kernels store every
+      // element once, and clearing the tensor first is one more pass over it (537 MB at (1,8,4096,64)).
+      const bool summed = (bias.sb == 0 && c.batch > 1) || (bias.sh == 0 && c.heads > 1);
+      dbias = (summed || c.causal) ? at::zeros_like(bias.t) : at::empty_like(bias.t);
+    }
     View t[8];
     if (packed) {
       if (!in_place_view(go, &t[4])) {

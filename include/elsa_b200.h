@@ -289,8 +289,9 @@ int elsa_row_stats(const void* q, const void* k,
  * (attention_bwd.py:188-224, 309-412, 415-527, 529-624) made by `twopass_attention_backward`
  * and `_dense_bias_backward` (attention_bwd.py:765-838, 939-970).
  * dbias is fp32, addressed with the dbias_stride_* like bias; where a stride is 0 the
- * contributions of that axis are summed (atomically).  The caller ALWAYS zeroes dbias before the call: besides
- * the sums, entries of pairs that the causal rule or the sequence length excludes are never written.
+ * contributions of that axis are summed (atomically).  The caller zeroes dbias before the call where an axis is summed
+ * or is_causal is set (entries of pairs that the causal rule excludes are never written); without either, every entry
+ * is stored.
  * workspace: elsa_backward_workspace_bytes (row_d, row_lse; on the tensor-core path also the fp32 dQ accumulator
  * for 16-bit inputs, or the 16-bit planes of q, dout, k, v for fp32 inputs). */
 int64_t elsa_backward_workspace_bytes(int dtype, int batch, int heads, int n_ctx, int head_dim,
