@@ -32,11 +32,20 @@ using namespace tc;
 
 namespace {
 
-constexpr int kSlots = 8;
+constexpr int kSlotsMax = 8;
 constexpr int kTileBytes = 128 * 64 * 2;                     // one 128 x 64 16-bit tile
-constexpr int kFoldWSmem = (2 + kSlots) * kTileBytes + 1024;  // + alignment slack
+// bias staging (rows must be contiguous): every fold warp has its own 32 rows x 32 keys; the 16-byte piece p of row r sits at piece p ^ (r & 7), so
+// that eight rows read at the same key touch 32 different banks
+constexpr int kBiasWarpFloats = 32 * 32;
 constexpr int kFoldWarps = 16, kFoldThreads = kFoldWarps * 32;
 constexpr int kThreads = kFoldThreads + 64;
+// BIAS: 0 none (64 < d <= 128), 1 biased with d <= 64, 2 biased with d > 64
+constexpr int fold_w_halves(int bias) { return bias == 1 ? 1 : 2; }
+constexpr int fold_w_bias_bufs(int bias) { return bias == 0 ? 0 : bias == 1 ? 2 : 1; }   // key tiles of bias in shared memory
+constexpr int fold_w_slots(int bias) { return bias == 0 ? kSlotsMax : bias == 1 ? 4 : 6; }
+constexpr int fold_w_smem(int bias) {
+  return (fold_w_halves(bias) + fold_w_slots(bias)) * kTileBytes + fold_w_bias_bufs(bias) * kFoldWarps * kBiasWarpFloats * 4 + 1024;   // + alignment slack
+}
 constexpr uint32_t kTmemCols = 512;
 constexpr int kProducerWarp = 16, kIssuerWarp = 17;
 constexpr float kRescaleThreshold = 8.0f;
@@ -47,11 +56,18 @@ struct FoldWParams {
   float* m; float* z; void* s;
   int n_ctx, q_start, q_len, part_width, n_parts, bh, heads, is_causal, summary_dtype;
   int n_keys, key_offset, head_dim;
-  int n_halves;                                 // 1 when head_dim <= 64 (biased problems), else 2
   float scale_log2;
   const float* bias; int64_t bsb, bsh, bsq, bsk;  // additive bias [.., N, N] (natural-log units) or null
+  int bias_stage;                               // 0: read the bias row by row; 1, 4: staged, 1 or 4 floats per copy
   int* status;
 };
+
+// asynchronous copy global -> shared of BYTES, of which the first `valid` are read and the rest become zeros
+template <int BYTES>
+__device__ __forceinline__ void cp_async(uint32_t dst, const float* src, int valid) {
+  if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+}
 
 __device__ __forceinline__ float max3w(float a, float b, float c) {
   float d;
@@ -78,12 +94,13 @@ __device__ __forceinline__ void store_row16(TS* dst, const float* v, int n) {
   }
 }
 
-template <typename T, bool BIAS>
+template <typename T, int BIAS>
 __global__ void __launch_bounds__(kThreads, 1)
 fold_tcw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const FoldWParams prm) {
+  constexpr int kSlots = fold_w_slots(BIAS), kHalves = fold_w_halves(BIAS), kBiasBufs = fold_w_bias_bufs(BIAS);
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bars[2 * kSlots + 9];
+  __shared__ __align__(8) uint64_t bars[2 * kSlotsMax + 9];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
   __shared__ float row_max[2][4][128];   // [key-tile parity][column quarter][row]: the quarter-row maxima
@@ -107,7 +124,7 @@ fold_tcw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   auto sQ = [&](int h) { return smem_base + h * kTileBytes; };
-  auto sSlot = [&](int i) { return smem_base + (2 + i) * kTileBytes; };
+  auto sSlot = [&](int i) { return smem_base + (kHalves + i) * kTileBytes; };
   const uint32_t bar0 = smem_u32(bars);
   const uint32_t bar_q = bar0;
   auto bar_full = [&](int i) { return bar0 + 8 * (1 + i); };
@@ -143,9 +160,8 @@ fold_tcw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     if (n_t > 0 && lane == 0) {
       // ---------------- TMA producer ----------------
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
-      const int nh = BIAS ? prm.n_halves : 2;
-      mbar_arrive_expect_tx(bar_q, nh * kTileBytes);
-      for (int h = 0; h < nh; ++h) tma_load_4d(sQ(h), &tmap_q, bar_q, 64 * h, q0, hi, bi);
+      mbar_arrive_expect_tx(bar_q, kHalves * kTileBytes);
+      for (int h = 0; h < kHalves; ++h) tma_load_4d(sQ(h), &tmap_q, bar_q, 64 * h, q0, hi, bi);
       int seq = 0;
       bool ok = true;
       auto load = [&](const CUtensorMap* map, int tile, int half) {
@@ -155,11 +171,11 @@ fold_tcw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         tma_load_4d(sSlot(slot), map, bar_full(slot), 64 * half, k_begin + tile * 128, hi, bi);
         ++seq;
       };
-      for (int h = 0; h < nh && ok; ++h) load(&tmap_k, 0, h);
+      for (int h = 0; h < kHalves && ok; ++h) load(&tmap_k, 0, h);
       for (int j = 0; j < n_t && ok; ++j) {
         if (j + 1 < n_t)
-          for (int h = 0; h < nh && ok; ++h) load(&tmap_k, j + 1, h);
-        for (int h = 0; h < nh && ok; ++h) load(&tmap_v, j, h);
+          for (int h = 0; h < kHalves && ok; ++h) load(&tmap_k, j + 1, h);
+        for (int h = 0; h < kHalves && ok; ++h) load(&tmap_v, j, h);
       }
     }
   } else if (warp_u == kIssuerWarp) {
@@ -173,10 +189,9 @@ fold_tcw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const uint64_t dk_slot0 = make_sdesc(sSlot(0), 16, 1024), dv_slot0 = make_sdesc(sSlot(0), 128 * 128, 1024);
       constexpr uint64_t kSlotStep = kTileBytes >> 4;   // descriptor address field counts 16-byte units
       int seq = 0;
-      const int nh = BIAS ? prm.n_halves : 2;
       bool ok = mbar_wait_warp(bar_q, 0, &abort_flag, prm.status, BAR_Q);
       auto issue_s = [&]() {
-        for (int h = 0; h < nh && ok; ++h) {
+        for (int h = 0; h < kHalves && ok; ++h) {
           const int slot = seq % kSlots;
           if (!(ok = mbar_wait_warp(bar_full(slot), (seq / kSlots) & 1, &abort_flag, prm.status, BAR_FULL))) return;
           tc_fence_after();
@@ -198,7 +213,7 @@ fold_tcw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (!(ok = mbar_wait_warp(bar_p, j & 1, &abort_flag, prm.status, BAR_P))) break;
         tc_fence_after();
         // O_lo, O_hi of this key tile start from zero (the fold warps took the previous ones into their registers)
-        for (int h = 0; h < nh && ok; ++h) {
+        for (int h = 0; h < kHalves && ok; ++h) {
           const int slot = seq % kSlots;
           if (!(ok = mbar_wait_warp(bar_full(slot), (seq / kSlots) & 1, &abort_flag, prm.status, BAR_FULL))) break;
           tc_fence_after();
@@ -218,8 +233,8 @@ fold_tcw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const int qi = q0 + row;
     const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
     const float c = prm.scale_log2;
-    const bool two_halves = BIAS ? prm.n_halves == 2 : true;   // (warp-uniform: tcgen05.ld is collective; unbiased problems here are wide)
-    constexpr bool has_bias = BIAS;
+    constexpr bool two_halves = kHalves == 2;
+    constexpr bool has_bias = BIAS != 0;
     // with a bias the scores are moved to the log2 domain at once (s c + b log2 e) and the scale below becomes 1
     const float cc = has_bias ? 1.f : c;
     const float* bias_row = has_bias ? prm.bias + bi * prm.bsb + hi * prm.bsh + static_cast<int64_t>(min(qi, prm.n_ctx - 1)) * prm.bsq : nullptr;
@@ -243,8 +258,41 @@ fold_tcw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
     };
 
+    // The bias of a key tile: each warp copies its own 32 rows x 32 keys into shared memory with whole 128-byte row pieces
+    // (one row per instruction, or four where rows are 16-byte aligned), a tile ahead, and a thread then reads its row.
+    // Loads by the thread itself put a warp's 32 rows into every instruction, i.e. 32 cache lines, and the fold waited for
+    // them: fp16 (1,8,4096,64) with a per-head bias, 192 us for the forward with one tile of staging, 147 with two (and no
+    // prefetch into L2, whose 32 lines per instruction cost more than they gain: 161).
+    float* stage0 = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)) + (kHalves + kSlots) * kTileBytes) + warp * kBiasWarpFloats;
+    auto stage_of = [&](int j) { return stage0 + (kBiasBufs == 2 ? j & 1 : 0) * kFoldWarps * kBiasWarpFloats; };
+    const float* bias_bh = has_bias ? prm.bias + bi * prm.bsb + hi * prm.bsh : nullptr;
+    auto stage_bias = [&](int j) {
+      const int k0 = k_begin + j * 128 + 32 * cq, w0 = q0 + qd * 32;     // first (local) key and first row of the warp's piece
+      float* stage = stage_of(j);
+      if (j >= n_t) { asm volatile("cp.async.commit_group;" ::: "memory"); return; }   // (keeps the count of groups)
+      if (prm.bias_stage == 4) {
+        const int c4 = (lane & 7) * 4, valid = max(0, min(4, k_end - k0 - c4)) * 4;
+        const float* src = bias_bh + (valid > 0 ? k0 + koff + c4 : 0);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = 4 * i + (lane >> 3);
+          cp_async<16>(smem_u32(stage + r * 32 + (c4 ^ ((r & 7) << 2))), src + static_cast<int64_t>(min(w0 + r, prm.n_ctx - 1)) * prm.bsq, valid);
+        }
+      } else {
+        const int valid = k0 + lane < k_end ? 4 : 0;
+        const float* src = bias_bh + (valid > 0 ? k0 + koff + lane : 0);
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r)
+          cp_async<4>(smem_u32(stage + r * 32 + (lane ^ ((r & 7) << 2))), src + static_cast<int64_t>(min(w0 + r, prm.n_ctx - 1)) * prm.bsq, valid);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (BIAS && prm.bias_stage) {
+      for (int j = 0; j < kBiasBufs; ++j) stage_bias(j);
+    }
+
     for (int j = 0; j < n_t; ++j) {
-      if constexpr (BIAS) {
+      if (BIAS != 0 && !prm.bias_stage) {
         // this thread's 128 bytes of the bias row for the NEXT key tile: on their way into L2 while this tile is folded
         const int kn = k_begin + (j + 1) * 128 + 32 * cq;
         if (kn + 32 <= k_end) {
@@ -266,19 +314,21 @@ fold_tcw_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       tc_fence_before();
       mbar_arrive_warp(bar_sfree, lane);        // S may be overwritten with the next tile's scores
       const int k0 = k_begin + j * 128 + 32 * cq;           // first (local) key of this thread's columns
-      if constexpr (BIAS) {
-        const float* bp = bias_row + static_cast<int64_t>(k0 + koff) * prm.bsk;
-        if (prm.bsk == 1 && k0 + 32 <= k_end && (reinterpret_cast<uintptr_t>(bp) & 31u) == 0) {
-          // the thread's 128 bytes of the bias row as four whole sectors (a warp's 32 rows are 32 different lines:
-          // 4-byte loads would fetch every sector eight times)
+      if constexpr (BIAS != 0) {
+        if (prm.bias_stage) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(kBiasBufs > 0 ? kBiasBufs - 1 : 0) : "memory");
+          __syncwarp();
+          const float* stage = stage_of(j);
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            float b8[8];
-            ld_global_v8(bp + 8 * g, b8);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sv[8 * g + e] = fmaf(sv[8 * g + e], c, b8[e] * 1.4426950408889634f);
+          for (int g = 0; g < 8; ++g) {
+            const float4 b = *reinterpret_cast<const float4*>(stage + lane * 32 + ((4 * g) ^ ((lane & 7) << 2)));
+            sv[4 * g] = fmaf(sv[4 * g], c, b.x * 1.4426950408889634f); sv[4 * g + 1] = fmaf(sv[4 * g + 1], c, b.y * 1.4426950408889634f);
+            sv[4 * g + 2] = fmaf(sv[4 * g + 2], c, b.z * 1.4426950408889634f); sv[4 * g + 3] = fmaf(sv[4 * g + 3], c, b.w * 1.4426950408889634f);
           }
+          __syncwarp();                           // every lane has read its row: the buffer takes the next tile
+          stage_bias(j + kBiasBufs);
         } else {
+          const float* bp = bias_row + static_cast<int64_t>(k0 + koff) * prm.bsk;
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             const float b = (k0 + i < k_end) ? bp[i * prm.bsk] : 0.f;
@@ -412,17 +462,21 @@ int fold_tcw(const FoldParams& p, int dtype, cudaStream_t st) {
   prm.n_parts = p.n_parts; prm.bh = p.bh; prm.heads = p.heads; prm.is_causal = p.is_causal; prm.summary_dtype = p.summary_dtype;
   prm.n_keys = p.n_keys; prm.key_offset = p.key_offset; prm.head_dim = p.head_dim;
   prm.scale_log2 = p.scale_log2;
-  prm.n_halves = p.head_dim > 64 ? 2 : 1;
   prm.bias = p.bias; prm.bsb = p.bsb; prm.bsh = p.bsh; prm.bsq = p.bsq; prm.bsk = p.bsk;
+  // 16-byte copies need every row piece on a 16-byte boundary (pieces start at multiples of 32 keys from key_offset)
+  const bool by16 = (reinterpret_cast<uintptr_t>(p.bias) & 15u) == 0 && ((p.bsb | p.bsh | p.bsq | p.key_offset) & 3) == 0;
+  prm.bias_stage = !p.bias || p.bsk != 1 ? 0 : by16 ? 4 : 1;
   dim3 grid(static_cast<unsigned>((p.q_len + 127) / 128), static_cast<unsigned>(p.n_parts), static_cast<unsigned>(p.bh));
-  auto launch = [&](auto kernel) -> int {
-    const int r = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kFoldWSmem);
+  const int form = !p.bias ? 0 : p.head_dim <= 64 ? 1 : 2, smem = fold_w_smem(form);
+  auto launch = [&](auto k0, auto k1, auto k2) -> int {
+    const auto kernel = form == 0 ? k0 : form == 1 ? k1 : k2;
+    const int r = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     if (r != ELSA_OK) return r;
-    kernel<<<grid, kThreads, kFoldWSmem, st>>>(mq, mk, mv, prm);
+    kernel<<<grid, kThreads, smem, st>>>(mq, mk, mv, prm);
     return ELSA_OK;
   };
-  if (dtype == ELSA_F16) rc = p.bias ? launch(&fold_tcw_kernel<__half, true>) : launch(&fold_tcw_kernel<__half, false>);
-  else rc = p.bias ? launch(&fold_tcw_kernel<__nv_bfloat16, true>) : launch(&fold_tcw_kernel<__nv_bfloat16, false>);
+  if (dtype == ELSA_F16) rc = launch(&fold_tcw_kernel<__half, 0>, &fold_tcw_kernel<__half, 1>, &fold_tcw_kernel<__half, 2>);
+  else rc = launch(&fold_tcw_kernel<__nv_bfloat16, 0>, &fold_tcw_kernel<__nv_bfloat16, 1>, &fold_tcw_kernel<__nv_bfloat16, 2>);
   if (rc != ELSA_OK) return rc;
   ELSA_LAUNCH_CHECK();
   return ELSA_OK;
