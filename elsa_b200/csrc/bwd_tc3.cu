@@ -10,12 +10,12 @@
 // streamed dQ (one kernel, five contractions) would need global atomics for dQ and more TMEM than there is, so the
 // work is done by two kernels of the same shape as the forward one, seven contractions per pair in all:
 //
-//   bwd3_dq_kernel    one CTA per 128-row QUERY tile, 128-key tiles streamed:
+//   bwd3_dq_body      one CTA per 128-row QUERY tile, 128-key tiles streamed:
 //                       S  = Q K^T, dP = dO V^T       A = Q / dO planes (shared memory), B = K / V planes
 //                       dS = P (dP - D), P = 2^(S c - LSE)          four threads per query row
 //                       dQ_j = dS K                    A = dS planes (TMEM), B = the same K planes, MN-major
 //                     dQ = scale * sum_j dQ_j in registers, written once: no atomics, deterministic
-//   bwd3_dkv_kernel   one CTA per 128-row KEY tile, 64-query tiles streamed:
+//   bwd3_dkv_body    one CTA per 128-row KEY tile, 64-query tiles streamed:
 //                       S^T = K Q^T, dP^T = V dO^T     A = K / V planes (shared memory), B = Q / dO planes
 //                       P^T, dS^T                      four threads per key row; -LSE, -D of the tile's queries
 //                                                      arrive with the tile (bulk copies into a small ring)
@@ -27,6 +27,8 @@
 // consumes them (planes from the lightest to the leading one: the cross terms are added in order of increasing
 // weight).  The score / dP tiles of pair t+1 are issued as soon as the fold warps hold those of pair t in registers,
 // so the exponentials and the splits of one pair overlap the contractions of its neighbours.
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "tc_common.cuh"
 
@@ -125,10 +127,8 @@ __device__ __forceinline__ float abs_max16(const float* x) {
 // dQ_j has read them, while S of tile j+1 needs the next three) | V ring, 2 slots
 // ------------------------------------------------------------------------------------------------------------------
 template <bool BIAS>
-__global__ void __launch_bounds__(kThreads, 1)
-bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
-               const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-               const Bwd3Params prm) {
+__device__ __forceinline__ void bwd3_dq_body(const CUtensorMap& tmap_q, const CUtensorMap& tmap_do, const CUtensorMap& tmap_k,
+                    const CUtensorMap& tmap_v, const Bwd3Params& prm) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * (kDqKSlots + kDqVSlots) + 9];
   __shared__ uint32_t tmem_base_slot;
@@ -138,7 +138,10 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.y;
-  const int q0 = blockIdx.x * 128;
+  const int n_qt = (prm.n_ctx + 127) / 128;
+  if (static_cast<int>(blockIdx.x) >= n_qt) return;
+  // causal: a tile's work grows with its first row, so the long ones are handed out first
+  const int q0 = (prm.is_causal ? n_qt - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x)) * 128;
   const int N = prm.n_ctx, NK = prm.n_keys, koff = prm.key_offset;
   int ke = NK;
   if (prm.is_causal) ke = min(ke, min(q0 + 128, N) - koff);   // keys above the tile's last row are never admissible
@@ -420,10 +423,8 @@ bwd3_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
 // TMEM columns: S^T [0,64) dP^T [64,128) P^T planes [128,224) dS^T planes [224,320) dV_i [320,384) dK_i [384,448)
 // ------------------------------------------------------------------------------------------------------------------
 template <bool BIAS>
-__global__ void __launch_bounds__(kThreads, 1)
-bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
-                const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                const Bwd3Params prm) {
+__device__ __forceinline__ void bwd3_dkv_body(const CUtensorMap& tmap_q, const CUtensorMap& tmap_do, const CUtensorMap& tmap_k,
+                    const CUtensorMap& tmap_v, const Bwd3Params& prm) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * kKvSlots + 9];
   __shared__ uint32_t tmem_base_slot;
@@ -434,6 +435,7 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.y;
   const int k0 = blockIdx.x * 128;                  // first (local) key row of this CTA
+  if (k0 >= prm.n_keys) return;
   const int N = prm.n_ctx, NK = prm.n_keys;
   const int kseq0 = k0 + prm.key_offset;            // its index in the sequence
   const int n_q64 = (N + 63) / 64;
@@ -712,6 +714,17 @@ bwd3_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (warp == kProducerWarp) tmem_dealloc(tmem_base, kTmemCols);
 }
 
+// Both bodies in one launch, the longer CTAs (dK / dV, blockIdx.z == 0) first: as two launches each ended in a nearly empty
+// wave of its own (fp32 (1,8,4096,64) 402 -> 392 us).
+template <bool BIAS>
+__global__ void __launch_bounds__(kThreads, 1)
+bwd3_kernel(const __grid_constant__ CUtensorMap tmap_q128, const __grid_constant__ CUtensorMap tmap_do128,
+            const __grid_constant__ CUtensorMap tmap_q64, const __grid_constant__ CUtensorMap tmap_do64,
+            const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const Bwd3Params prm) {
+  if (blockIdx.z == 0) bwd3_dkv_body<BIAS>(tmap_q64, tmap_do64, tmap_k, tmap_v, prm);
+  else bwd3_dq_body<BIAS>(tmap_q128, tmap_do128, tmap_k, tmap_v, prm);
+}
+
 }  // namespace
 
 bool bwd_tc3_supported(int dtype, int head_dim, bool has_bias) { return fold_tc3_supported(dtype, head_dim, has_bias); }
@@ -771,17 +784,15 @@ int bwd_tc3(const BwdParams& p, const void* out, Strides os, const float* row_m,
   } else {
     mk128 = mv128 = mq64;   // never dereferenced: no key tile is visited
   }
-  const dim3 qgrid(static_cast<unsigned>((N + 127) / 128), static_cast<unsigned>(bh));
-  const dim3 kgrid(static_cast<unsigned>((NK + 127) / 128), static_cast<unsigned>(bh));
-  auto launch = [&](auto dq_kernel, auto dkv_kernel) -> int {
-    int r;
-    if ((r = ensure_dynamic_smem(reinterpret_cast<const void*>(dq_kernel), kDqSmem)) != ELSA_OK) return r;
-    if ((r = ensure_dynamic_smem(reinterpret_cast<const void*>(dkv_kernel), kKvSmem)) != ELSA_OK) return r;
-    dq_kernel<<<qgrid, kThreads, kDqSmem, st>>>(mq128, mdo128, mk128, mv128, prm);
-    if (NK > 0) dkv_kernel<<<kgrid, kThreads, kKvSmem, st>>>(mq64, mdo64, mk128, mv128, prm);
+  const dim3 grid(static_cast<unsigned>((std::max(N, NK) + 127) / 128), static_cast<unsigned>(bh), 2u);
+  constexpr int kSmem = std::max(kDqSmem, kKvSmem);
+  auto launch = [&](auto kernel) -> int {
+    const int r = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kSmem);
+    if (r != ELSA_OK) return r;
+    kernel<<<grid, kThreads, kSmem, st>>>(mq128, mdo128, mq64, mdo64, mk128, mv128, prm);
     return ELSA_OK;
   };
-  rc = p.bias ? launch(&bwd3_dq_kernel<true>, &bwd3_dkv_kernel<true>) : launch(&bwd3_dq_kernel<false>, &bwd3_dkv_kernel<false>);
+  rc = launch(p.bias ? &bwd3_kernel<true> : &bwd3_kernel<false>);
   if (rc != ELSA_OK) return rc;
   ELSA_LAUNCH_CHECK();
   return ELSA_OK;

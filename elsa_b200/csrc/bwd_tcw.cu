@@ -8,11 +8,11 @@
 // that no longer fits, so the work is split the way the fp32 backward is (bwd_tc3.cu), seven contractions per tile
 // pair, no atomics:
 //
-//   bwdw_dq_kernel    one CTA per 128-row QUERY tile, 128-key tiles streamed:
+//   bwdw_dq_body      one CTA per 128-row QUERY tile, 128-key tiles streamed:
 //                       S  = Q_lo K_lo^T + Q_hi K_hi^T,  dP = dO_lo V_lo^T + dO_hi V_hi^T        (N = 128)
 //                       dS = P (dP - D), P = 2^(S c - LSE), rounded to the input type, into TMEM
 //                       dQ_h += dS K_h, h = lo, hi       accumulated in TMEM over the key tiles  (N = 64 each)
-//   bwdw_dkv_kernel   one CTA per 128-row KEY tile, 64-query tiles streamed:
+//   bwdw_dkv_body    one CTA per 128-row KEY tile, 64-query tiles streamed:
 //                       S^T = K_lo Q_lo^T + K_hi Q_hi^T, dP^T = V_lo dO_lo^T + V_hi dO_hi^T      (N = 64)
 //                       P^T, dS^T rounded to the input type, into TMEM
 //                       dV_h += P^T dO_h, dK_h += dS^T Q_h   accumulated in TMEM over the query tiles
@@ -20,6 +20,7 @@
 // Gradients accumulate in TMEM (the 16-bit outputs do not see the tensor core's truncating accumulation; the fp32
 // kernels keep their running sums in registers for that reason).  Both kernels: 16 fold warps (four threads per row),
 // a TMA producer warp, an MMA-issuing warp; all waits bounded.
+#include <algorithm>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -97,10 +98,8 @@ __device__ __forceinline__ void store16(TO* dst, const uint32_t (&r)[16], float 
 // TMEM columns: S [0,128) dP [128,256) dQ_lo [256,320) dQ_hi [320,384) dS [384,448)
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T, bool BIAS>
-__global__ void __launch_bounds__(kThreads, 1)
-bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
-               const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-               const BwdWParams prm) {
+__device__ __forceinline__ void bwdw_dq_body(const CUtensorMap& tmap_q, const CUtensorMap& tmap_do, const CUtensorMap& tmap_k,
+                    const CUtensorMap& tmap_v, const BwdWParams& prm) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * (kDqKSlots + kDqVSlots) + 5];
   __shared__ uint32_t tmem_base_slot;
@@ -110,7 +109,10 @@ bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // (known to be warp-uniform)
   const int bh = blockIdx.y;
   const int bi = bh / prm.heads, hi = bh - bi * prm.heads;   // tensor-map coordinates of this (batch*head)
-  const int q0 = blockIdx.x * 128;
+  const int n_qt = (prm.n_ctx + 127) / 128;
+  if (static_cast<int>(blockIdx.x) >= n_qt) return;
+  // causal: a tile's work grows with its first row, so the long ones are handed out first
+  const int q0 = (prm.is_causal ? n_qt - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x)) * 128;
   const int N = prm.n_ctx, NK = prm.n_keys, koff = prm.key_offset;
   int ke = NK;
   if (prm.is_causal) ke = min(ke, min(q0 + 128, N) - koff);   // keys above the tile's last row are never admissible
@@ -368,10 +370,8 @@ bwdw_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
 // TMEM columns: S^T [0,64) dP^T [64,128) P^T [128,160) dS^T [160,192) dV_lo dV_hi [192,320) dK_lo dK_hi [320,448)
 // ------------------------------------------------------------------------------------------------------------------
 template <typename T, bool BIAS>
-__global__ void __launch_bounds__(kThreads, 1)
-bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_do,
-                const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                const BwdWParams prm) {
+__device__ __forceinline__ void bwdw_dkv_body(const CUtensorMap& tmap_q, const CUtensorMap& tmap_do, const CUtensorMap& tmap_k,
+                    const CUtensorMap& tmap_v, const BwdWParams& prm) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bars[2 * kKvSlots + 5];
   __shared__ uint32_t tmem_base_slot;
@@ -382,6 +382,7 @@ bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const int bh = blockIdx.y;
   const int bi = bh / prm.heads, hi = bh - bi * prm.heads;   // tensor-map coordinates of this (batch*head)
   const int k0 = blockIdx.x * 128;                  // first (local) key row of this CTA
+  if (k0 >= prm.n_keys) return;
   const int N = prm.n_ctx, NK = prm.n_keys;
   const int kseq0 = k0 + prm.key_offset;            // its index in the sequence
   const int n_q64 = (N + 63) / 64;
@@ -621,6 +622,17 @@ bwdw_dkv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (warp == kProducerWarp) tmem_dealloc(tmem_base, kTmemCols);
 }
 
+// Both bodies in one launch, the longer CTAs (dK / dV, blockIdx.z == 0) first: as two launches each ended in a nearly empty
+// wave of its own (fwd+bwd of fp16 (1,8,8192,128) 1457 -> 1369 us).
+template <typename T, bool BIAS>
+__global__ void __launch_bounds__(kThreads, 1)
+bwdw_kernel(const __grid_constant__ CUtensorMap tmap_q128, const __grid_constant__ CUtensorMap tmap_do128,
+            const __grid_constant__ CUtensorMap tmap_q64, const __grid_constant__ CUtensorMap tmap_do64,
+            const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const BwdWParams prm) {
+  if (blockIdx.z == 0) bwdw_dkv_body<T, BIAS>(tmap_q64, tmap_do64, tmap_k, tmap_v, prm);
+  else bwdw_dq_body<T, BIAS>(tmap_q128, tmap_do128, tmap_k, tmap_v, prm);
+}
+
 // -D = -sum_d out*dout, -LSE = -(m + log2(max(z, 1e-30))) into the padded layout; padding: -D = 0, -LSE = -inf
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -709,17 +721,15 @@ static int bwd_tcw_t(const BwdParams& p, const void* out, Strides os, const floa
   } else {
     mk128 = mv128 = mq64;   // never dereferenced: no key tile is visited
   }
-  const dim3 qgrid(static_cast<unsigned>((N + 127) / 128), static_cast<unsigned>(bh));
-  const dim3 kgrid(static_cast<unsigned>((NK + 127) / 128), static_cast<unsigned>(bh));
-  auto launch = [&](auto dq_kernel, auto dkv_kernel) -> int {
-    int r;
-    if ((r = ensure_dynamic_smem(reinterpret_cast<const void*>(dq_kernel), kDqSmem)) != ELSA_OK) return r;
-    if ((r = ensure_dynamic_smem(reinterpret_cast<const void*>(dkv_kernel), kKvSmem)) != ELSA_OK) return r;
-    dq_kernel<<<qgrid, kThreads, kDqSmem, st>>>(mq128, mdo128, mk128, mv128, prm);
-    if (NK > 0) dkv_kernel<<<kgrid, kThreads, kKvSmem, st>>>(mq64, mdo64, mk128, mv128, prm);
+  const dim3 grid(static_cast<unsigned>((std::max(N, NK) + 127) / 128), static_cast<unsigned>(bh), 2u);
+  constexpr int kSmem = std::max(kDqSmem, kKvSmem);
+  auto launch = [&](auto kernel) -> int {
+    const int r = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kSmem);
+    if (r != ELSA_OK) return r;
+    kernel<<<grid, kThreads, kSmem, st>>>(mq128, mdo128, mq64, mdo64, mk128, mv128, prm);
     return ELSA_OK;
   };
-  rc = p.bias ? launch(&bwdw_dq_kernel<T, true>, &bwdw_dkv_kernel<T, true>) : launch(&bwdw_dq_kernel<T, false>, &bwdw_dkv_kernel<T, false>);
+  rc = launch(p.bias ? &bwdw_kernel<T, true> : &bwdw_kernel<T, false>);
   if (rc != ELSA_OK) return rc;
   ELSA_LAUNCH_CHECK();
   return ELSA_OK;
