@@ -75,6 +75,24 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint
                ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar) : "memory");
 }
 
+// packed pairs (fma.f32x2 and friends) over register arrays
+__device__ __forceinline__ float2 pair_of(const uint32_t* r, int i) { return make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])); }
+template <int N>
+__device__ __forceinline__ void scale_by(float (&x)[N], float f) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const float2 v = __fmul2_rn(make_float2(x[i], x[i + 1]), make_float2(f, f));
+    x[i] = v.x; x[i + 1] = v.y;
+  }
+}
+__device__ __forceinline__ void add_scaled16(float (&sum)[16], const uint32_t (&r)[16], float f) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 2) {
+    const float2 v = __ffma2_rn(pair_of(r, i), make_float2(f, f), make_float2(sum[i], sum[i + 1]));
+    sum[i] = v.x; sum[i + 1] = v.y;
+  }
+}
+
 // the first n (a multiple of 4, possibly <= 0) of 16 consecutive values of a gradient row
 __device__ __forceinline__ void store16(float* dst, const float (&v)[16], float f, int n) {
 #pragma unroll
@@ -307,8 +325,7 @@ __device__ __forceinline__ void bwd3_dq_body(const CUtensorMap& tmap_q, const CU
       uint32_t r[16];
       tmem_ld16(tdQ + lane_off + 16 * cq, r);
       tmem_wait_ld();
-#pragma unroll
-      for (int i = 0; i < 16; ++i) dq_run[i] = fmaf(__uint_as_float(r[i]), inv_r, dq_run[i]);
+      add_scaled16(dq_run, r, inv_r);
     };
 
     for (int j = 0; alive && j < n_t; ++j) {
@@ -346,11 +363,18 @@ __device__ __forceinline__ void bwd3_dq_body(const CUtensorMap& tmap_q, const CU
               if (kb + i < NK) ab[i] = fmaf(bp[i * prm.bsk], 1.4426950408889634f, nlse);
           }
         }
+        // (packed pairs and a mask loop of its own: the fold warps issue in 50 to 64 % of the cycles, their instructions count)
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float p = fast_exp2(fmaf(__uint_as_float(rs[i]), c, ab[i]));
-          if (masked && kb + i > lim) p = 0.f;
-          ds[i] = p * fmaf(__uint_as_float(rp[i]), idp, nd);
+        for (int i = 0; i < 32; i += 2) {
+          const float2 x = __ffma2_rn(pair_of(rs, i), make_float2(c, c), make_float2(ab[i], ab[i + 1]));
+          const float2 t = __ffma2_rn(pair_of(rp, i), make_float2(idp, idp), make_float2(nd, nd));
+          const float2 d2 = __fmul2_rn(make_float2(fast_exp2(x.x), fast_exp2(x.y)), t);
+          ds[i] = d2.x; ds[i + 1] = d2.y;
+        }
+        if (masked) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (kb + i > lim) ds[i] = 0.f;
         }
         if constexpr (BIAS) {
           // dbias = dS (every (query, key) pair is visited exactly once by this kernel); pairs that the causal rule or
@@ -383,8 +407,7 @@ __device__ __forceinline__ void bwd3_dq_body(const CUtensorMap& tmap_q, const CU
         if (!mbar_wait_warp(bar_row(qd), j & 1, &abort_flag, prm.status, BAR_ROW)) { alive = false; break; }
         const float mx = fmaxf(fmaxf(row_max[j & 1][0][row], row_max[j & 1][1][row]), fmaxf(row_max[j & 1][2][row], row_max[j & 1][3][row]));
         r_scale = plane_scale(__float_as_uint(mx));
-#pragma unroll
-        for (int i = 0; i < 32; ++i) ds[i] *= r_scale;
+        scale_by(ds, r_scale);
       }
       if (j > 0) {
         // dQ of the previous key tile has retired: it goes into the running sum, and the dS planes are free
@@ -612,11 +635,8 @@ __device__ __forceinline__ void bwd3_dkv_body(const CUtensorMap& tmap_q, const C
       tmem_ld16(tdV + lane_off + 16 * cq, rv);
       tmem_ld16(tdK + lane_off + 16 * cq, rk);
       tmem_wait_ld();
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        dv_run[i] = fmaf(__uint_as_float(rv[i]), inv_v, dv_run[i]);
-        dk_run[i] = fmaf(__uint_as_float(rk[i]), inv_r, dk_run[i]);
-      }
+      add_scaled16(dv_run, rv, inv_v);
+      add_scaled16(dk_run, rk, inv_r);
     };
 
     for (int it = 0; it < n_it; ++it) {
@@ -657,17 +677,23 @@ __device__ __forceinline__ void bwd3_dkv_body(const CUtensorMap& tmap_q, const C
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           const float4 nl = nl4[g], nd = nd4[g];            // -LSE, -D of 4 queries (warp-wide broadcast reads)
-          const float nle[4] = {nl.x, nl.y, nl.z, nl.w}, nde[4] = {nd.x, nd.y, nd.z, nd.w};
+          const float2 nle[2] = {make_float2(nl.x, nl.y), make_float2(nl.z, nl.w)}, nde[2] = {make_float2(nd.x, nd.y), make_float2(nd.z, nd.w)};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = 4 * g + e;
-            float a = nle[e] + kLog2Unit;
-            if constexpr (BIAS) a += bb[i];
-            float pv = fast_exp2(fmaf(__uint_as_float(rs[i]), c, a));
-            if (masked && !(key_ok && (!prm.is_causal || qc + i >= key_seq))) pv = 0.f;
-            p[i] = pv;
-            ds[i] = pv * fmaf(__uint_as_float(rp[i]), idp, nde[e] * k2);
+          for (int e = 0; e < 2; ++e) {
+            const int i = 4 * g + 2 * e;
+            float2 a = __fadd2_rn(nle[e], make_float2(kLog2Unit, kLog2Unit));
+            if constexpr (BIAS) a = __fadd2_rn(a, make_float2(bb[i], bb[i + 1]));
+            const float2 x = __ffma2_rn(pair_of(rs, i), make_float2(c, c), a);
+            const float2 t = __ffma2_rn(pair_of(rp, i), make_float2(idp, idp), __fmul2_rn(nde[e], make_float2(k2, k2)));
+            const float2 pv = make_float2(fast_exp2(x.x), fast_exp2(x.y)), d2 = __fmul2_rn(pv, t);
+            p[i] = pv.x; p[i + 1] = pv.y;
+            ds[i] = d2.x; ds[i + 1] = d2.y;
           }
+        }
+        if (masked) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (!(key_ok && (!prm.is_causal || qc + i >= key_seq))) { p[i] = 0.f; ds[i] = 0.f; }
         }
       }
       float r_scale = 1.f;
@@ -678,8 +704,7 @@ __device__ __forceinline__ void bwd3_dkv_body(const CUtensorMap& tmap_q, const C
         if (!mbar_wait_warp(bar_row(qd), it & 1, &abort_flag, prm.status, BAR_ROW)) { alive = false; break; }
         const float mx = fmaxf(fmaxf(row_max[it & 1][0][row], row_max[it & 1][1][row]), fmaxf(row_max[it & 1][2][row], row_max[it & 1][3][row]));
         r_scale = plane_scale(__float_as_uint(mx));
-#pragma unroll
-        for (int i = 0; i < 16; ++i) ds[i] *= r_scale;
+        scale_by(ds, r_scale);
       }
       if (it > 0) {
         // dV, dK of the previous query tile have retired: they go into the running sums, and the planes are free

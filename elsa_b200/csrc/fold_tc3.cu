@@ -363,7 +363,10 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       tmem_ld16(tO + lane_off + 16 * cq, r);
       tmem_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 16; ++i) o_run[i] = fmaf(__uint_as_float(r[i]), iv, o_run[i]);
+      for (int i = 0; i < 16; i += 2) {
+        const float2 v = __ffma2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), make_float2(iv, iv), make_float2(o_run[i], o_run[i + 1]));
+        o_run[i] = v.x; o_run[i + 1] = v.y;
+      }
     };
 
     for (int j = 0; j < n_t; ++j) {
@@ -441,8 +444,9 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
         // ex2.approx: 2 units in the last place, i.e. 2.4e-7 relative on a weight
-        sv[i] = fast_exp2(fmaf(sv[i], cc, nm));
-        sv[i + 1] = fast_exp2(fmaf(sv[i + 1], cc, nm));
+        const float2 x = __ffma2_rn(make_float2(sv[i], sv[i + 1]), make_float2(cc, cc), make_float2(nm, nm));
+        sv[i] = fast_exp2(x.x);
+        sv[i + 1] = fast_exp2(x.y);
         ps[(i >> 1) & 3] += sv[i] + sv[i + 1];
       }
       zsum = zsum * alpha + ((ps[0] + ps[1]) + (ps[2] + ps[3]));

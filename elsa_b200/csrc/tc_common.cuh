@@ -358,8 +358,8 @@ __device__ __forceinline__ void split_planes_pair(float x0, float x1, uint32_t (
     w[kPlanes - 1] = *reinterpret_cast<const uint32_t*>(&a2);
   } else {
     const __half2 a0 = __floats2half2_rn(x0, x1);
-    const float2 f0 = __half22float2(a0);
-    const __half2 a1 = __floats2half2_rn(x0 - f0.x, x1 - f0.y);
+    const float2 r = __ffma2_rn(__half22float2(a0), make_float2(-1.f, -1.f), make_float2(x0, x1));   // exact
+    const __half2 a1 = __floats2half2_rn(r.x, r.y);
     w[0] = *reinterpret_cast<const uint32_t*>(&a0);
     w[1] = *reinterpret_cast<const uint32_t*>(&a1);
   }
