@@ -1,4 +1,4 @@
-"""Biased 16-bit problems at the edges of the bias staging: rows on 16-byte boundaries (N a multiple of 4) and off them, key
+"""Biased 16-bit problems at the edges of the bias staging (and short ones, on the kernels below it): rows on 16-byte boundaries (N a multiple of 4) and off them, key
 tails of one key up to a full tile, an offset base address, a broadcast and a dense bias, and the dense bias gradient, which
 the kernels store without a cleared tensor."""
 import pytest
@@ -9,7 +9,7 @@ import elsa_b200 as E
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [512, 513, 516, 639, 642, 772])
+@pytest.mark.parametrize("n", [7, 49, 64, 130, 512, 513, 516, 639, 642, 772])
 @pytest.mark.parametrize("d", [64, 40, 128])
 @pytest.mark.parametrize("kind", ["hnn", "bhnn", "offset"])
 @pytest.mark.parametrize("causal", [False, True])
