@@ -230,11 +230,18 @@ void bnhd_view(char* base, const Call& c, View* v) {
   v->st[2] = hd;
 }
 
+// A saved tensor as the backward may use it: saved-tensor hooks may return the values in another memory layout (a copy
+// built from the sizes alone, an unaligned slice), so nothing but the values is taken for granted.
+void check_unpacked(const at::Tensor& t, at::IntArrayRef sizes, at::ScalarType dtype, c10::Device dev) {
+  TORCH_CHECK(t.defined() && plain(t) && t.device() == dev && t.scalar_type() == dtype && t.sizes() == sizes,
+              "a saved tensor of the attention came back from its unpack hook with another shape, dtype or device");
+}
+
 struct AttentionBackward : public torch::autograd::Node {
   Call c{};
   bool packed = false, bias_grad = false;
-  at::ScalarType bias_dtype = at::kFloat;
-  std::vector<int64_t> bias_sizes;
+  at::ScalarType dtype = at::kFloat, bias_dtype = at::kFloat;
+  std::vector<int64_t> bias_sizes, bias_shape;      // of the caller's bias and of the canonical one
   SavedVariable q_, k_, v_, out_, state_, bias_;    // packed: q_ is the packed tensor, k_ and v_ stay empty
 
   std::string name() const override { return packed ? "TwopassAttentionQkvpackedBackward" : "TwopassAttentionBackward"; }
@@ -251,9 +258,21 @@ struct AttentionBackward : public torch::autograd::Node {
     if (!go.defined()) return result;
     at::AutoDispatchBelowADInplaceOrView below;
     at::Tensor q = q_.unpack(), out = out_.unpack(shared_from_this()), state = state_.unpack();
+    const int64_t B = c.batch, H = c.heads, N = c.n, D = c.d;
+    const std::array<int64_t, 5> packed_sizes{B, N, 3, H, D};
+    const std::array<int64_t, 4> sizes{B, H, N, D};
+    const c10::Device dev = go.device();
+    check_unpacked(q, packed ? at::IntArrayRef(packed_sizes) : at::IntArrayRef(sizes), dtype, dev);
+    check_unpacked(out, sizes, dtype, dev);
+    check_unpacked(state, {2 * padded_rows(c)}, at::kFloat, dev);
+    state = aligned(state);
     Bias bias;
     bias.t = bias_.unpack();
-    if (bias.t.defined()) bias_strides(&bias);
+    if (bias.t.defined()) {
+      check_unpacked(bias.t, bias_shape, at::kFloat, dev);
+      bias.t = bias.t.contiguous();
+      bias_strides(&bias);
+    }
     if (go.scalar_type() != q.scalar_type()) go = go.to(q.scalar_type());
     c10::cuda::CUDAGuard guard(q.device());
     at::Tensor dbias;
@@ -269,13 +288,19 @@ struct AttentionBackward : public torch::autograd::Node {
         go = aligned(go);
         in_place_view(go, &t[4]);
       }
+      q = aligned(q);
+      if (!in_place_view(out, &t[3])) {
+        out = aligned(out);
+        in_place_view(out, &t[3]);
+      }
       result[0] = new_tensor(q.sizes(), q, q.scalar_type());
       packed_views(data_of(q), c, q.element_size(), &t[0]);
-      bnhd_view(data_of(out), c, &t[3]);
       packed_views(data_of(result[0]), c, q.element_size(), &t[5]);
       run_backward(t, true, bias, dbias, state, c, q.device());
     } else {
       std::array<at::Tensor, 5> in{q, k_.unpack(), v_.unpack(), out, go};
+      check_unpacked(in[1], sizes, dtype, dev);
+      check_unpacked(in[2], sizes, dtype, dev);
       const bool strided = pick_layouts(in, t);
       for (int i = 0; i < 3; ++i) {
         result[i] = strided ? new_like_layout(in[i], t[i]) : new_tensor(q.sizes(), q, q.scalar_type());
@@ -307,10 +332,12 @@ std::shared_ptr<AttentionBackward> new_node(const Call& c, const at::Tensor& bia
   std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
   node->set_next_edges(torch::autograd::collect_next_edges(inputs..., bias));
   node->c = c;
+  node->dtype = c.dt == ELSA_F32 ? at::kFloat : c.dt == ELSA_F16 ? at::kHalf : at::kBFloat16;
   if (bias.defined()) {
     node->bias_grad = bias.requires_grad();
     node->bias_dtype = bias.scalar_type();
     node->bias_sizes = bias.sizes().vec();
+    node->bias_shape = canon.t.sizes().vec();
     node->bias_ = SavedVariable(canon.t, false);
   }
   return node;

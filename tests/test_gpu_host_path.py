@@ -1,0 +1,82 @@
+"""The native host path beside autograd's other machinery: what a user's program may put around a training call."""
+import pytest
+import torch
+
+import elsa_b200 as E
+from elsa_b200.attention_bwd import twopass_attention_qkvpacked
+
+pytestmark = pytest.mark.gpu
+
+ENTRIES = ["packed", "op"]
+
+
+def _problem(entry, n=130, dtype=torch.float16, bias=True, b=2, h=3, d=64):
+    """(inputs, bias or None, grad_out), no gradients asked for yet"""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+
+    def normal(*shape, dtype=dtype):
+        return torch.randn(shape, generator=gen, device="cuda").to(dtype)
+
+    inputs = [normal(b, n, 3, h, d)] if entry == "packed" else [normal(b, h, n, d) for _ in range(3)]
+    return inputs, normal(h, n, n, dtype=torch.float32) if bias else None, normal(b, h, n, d)
+
+
+def _call(entry, inputs, bias, **kwargs):
+    return (twopass_attention_qkvpacked if entry == "packed" else E.twopass_attention_train)(*inputs, bias=bias, **kwargs)
+
+
+def _leaves(inputs, bias):
+    inputs = [t.detach().requires_grad_(True) for t in inputs]
+    return inputs, None if bias is None else bias.detach().requires_grad_(True)
+
+
+def _gradients(entry, inputs, bias, grad_out):
+    inputs, bias = _leaves(inputs, bias)
+    out = _call(entry, inputs, bias)
+    return torch.autograd.grad(out, inputs + ([] if bias is None else [bias]), grad_out)
+
+
+def _assert_same(got, want):
+    # (dQ and summed bias gradients are added in arrival order; an element read from a wrong place gives errors of order 1)
+    for g, w in zip(got, want):
+        assert g.shape == w.shape and g.dtype == w.dtype
+        assert (g.double() - w.double()).norm() <= 1e-3 * w.double().norm()
+
+
+def _by_size(t):
+    return torch.empty(t.size(), dtype=t.dtype, device=t.device).copy_(t)
+
+
+def _off_alignment(t):
+    return torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].copy_(t.reshape(-1)).view(t.shape)
+
+
+def _transposed(t):
+    return t.transpose(-1, -2).contiguous().transpose(-1, -2) if t.dim() > 1 else t.clone()
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("n,dtype", [(49, torch.float16), (130, torch.float16), (130, torch.float32)])
+@pytest.mark.parametrize("hook", ["offload", "by_size", "off_alignment", "transposed"])
+def test_saved_tensors_may_come_back_in_another_layout(entry, n, dtype, hook):
+    inputs, bias, grad_out = _problem(entry, n, dtype)
+    want = _gradients(entry, inputs, bias, grad_out)
+    if hook == "offload":
+        hooks = torch.autograd.graph.save_on_cpu(pin_memory=True)
+    else:
+        pack = {"by_size": _by_size, "off_alignment": _off_alignment, "transposed": _transposed}[hook]
+        hooks = torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t)
+    with hooks:
+        got = _gradients(entry, inputs, bias, grad_out)
+    _assert_same(got, want)
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+def test_a_saved_tensor_of_another_kind_is_refused(entry):
+    inputs, bias, grad_out = _problem(entry)
+    for unpack in (lambda t: t.float(), lambda t: t.cpu(), lambda t: t[..., :1]):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            leaves, b = _leaves(inputs, bias)
+            out = _call(entry, leaves, b)
+        with pytest.raises(RuntimeError):
+            torch.autograd.grad(out, leaves, grad_out)
