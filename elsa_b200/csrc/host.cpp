@@ -251,30 +251,36 @@ struct AttentionBackward : public torch::autograd::Node {
     for (SavedVariable* s : {&q_, &k_, &v_, &out_, &state_, &bias_}) s->reset_data();
   }
 
+  struct Saved { at::Tensor q, k, v, out, state, bias; };   // packed: q is the packed tensor
+
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    variable_list result(packed ? 2 : 4);
-    at::Tensor go = grads[0];
-    if (!go.defined()) return result;
+    if (!grads[0].defined()) return variable_list(packed ? 2 : 4);
+    // Unpacking runs the user's hooks, with autograd in force: a checkpoint repeats the forward in there, and the repeated
+    // forward has to record and save what the first one did.
+    Saved s{q_.unpack(), k_.unpack(), v_.unpack(), out_.unpack(shared_from_this()), state_.unpack(), bias_.unpack()};
     at::AutoDispatchBelowADInplaceOrView below;
-    at::Tensor q = q_.unpack(), out = out_.unpack(shared_from_this()), state = state_.unpack();
+    return gradients(std::move(s), std::move(grads[0]));
+  }
+
+  variable_list gradients(Saved s, at::Tensor go) const {
+    variable_list result(packed ? 2 : 4);
     const int64_t B = c.batch, H = c.heads, N = c.n, D = c.d;
     const std::array<int64_t, 5> packed_sizes{B, N, 3, H, D};
     const std::array<int64_t, 4> sizes{B, H, N, D};
     const c10::Device dev = go.device();
-    check_unpacked(q, packed ? at::IntArrayRef(packed_sizes) : at::IntArrayRef(sizes), dtype, dev);
-    check_unpacked(out, sizes, dtype, dev);
-    check_unpacked(state, {2 * padded_rows(c)}, at::kFloat, dev);
-    state = aligned(state);
+    check_unpacked(s.q, packed ? at::IntArrayRef(packed_sizes) : at::IntArrayRef(sizes), dtype, dev);
+    check_unpacked(s.out, sizes, dtype, dev);
+    check_unpacked(s.state, {2 * padded_rows(c)}, at::kFloat, dev);
+    const at::Tensor state = aligned(s.state);
     Bias bias;
-    bias.t = bias_.unpack();
-    if (bias.t.defined()) {
-      check_unpacked(bias.t, bias_shape, at::kFloat, dev);
-      bias.t = bias.t.contiguous();
+    if (s.bias.defined()) {
+      check_unpacked(s.bias, bias_shape, at::kFloat, dev);
+      bias.t = s.bias.contiguous();
       bias_strides(&bias);
     }
-    if (go.scalar_type() != q.scalar_type()) go = go.to(q.scalar_type());
-    c10::cuda::CUDAGuard guard(q.device());
+    if (go.scalar_type() != dtype) go = go.to(dtype);
+    c10::cuda::CUDAGuard guard(dev);
     at::Tensor dbias;
     if (bias_grad) {
       // Sums over a broadcast axis and pairs that the causal rule leaves out need zeros.  Otherwise the kernels store every
@@ -288,25 +294,25 @@ struct AttentionBackward : public torch::autograd::Node {
         go = aligned(go);
         in_place_view(go, &t[4]);
       }
-      q = aligned(q);
-      if (!in_place_view(out, &t[3])) {
-        out = aligned(out);
-        in_place_view(out, &t[3]);
+      const at::Tensor q = aligned(s.q);
+      if (!in_place_view(s.out, &t[3])) {
+        s.out = aligned(s.out);
+        in_place_view(s.out, &t[3]);
       }
-      result[0] = new_tensor(q.sizes(), q, q.scalar_type());
+      result[0] = new_tensor(q.sizes(), q, dtype);
       packed_views(data_of(q), c, q.element_size(), &t[0]);
       packed_views(data_of(result[0]), c, q.element_size(), &t[5]);
-      run_backward(t, true, bias, dbias, state, c, q.device());
+      run_backward(t, true, bias, dbias, state, c, dev);
     } else {
-      std::array<at::Tensor, 5> in{q, k_.unpack(), v_.unpack(), out, go};
-      check_unpacked(in[1], sizes, dtype, dev);
-      check_unpacked(in[2], sizes, dtype, dev);
+      check_unpacked(s.k, sizes, dtype, dev);
+      check_unpacked(s.v, sizes, dtype, dev);
+      std::array<at::Tensor, 5> in{s.q, s.k, s.v, s.out, go};
       const bool strided = pick_layouts(in, t);
       for (int i = 0; i < 3; ++i) {
-        result[i] = strided ? new_like_layout(in[i], t[i]) : new_tensor(q.sizes(), q, q.scalar_type());
+        result[i] = strided ? new_like_layout(in[i], t[i]) : new_tensor(sizes, go, dtype);
         in_place_view(result[i], &t[5 + i]);
       }
-      run_backward(t, strided, bias, dbias, state, c, q.device());
+      run_backward(t, strided, bias, dbias, state, c, dev);
     }
     if (bias_grad) {
       dbias = dbias.view(bias_sizes);

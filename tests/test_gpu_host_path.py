@@ -1,6 +1,7 @@
 """The native host path beside autograd's other machinery: what a user's program may put around a training call."""
 import pytest
 import torch
+import torch.utils.checkpoint
 
 import elsa_b200 as E
 from elsa_b200.attention_bwd import twopass_attention_qkvpacked
@@ -80,3 +81,19 @@ def test_a_saved_tensor_of_another_kind_is_refused(entry):
             out = _call(entry, leaves, b)
         with pytest.raises(RuntimeError):
             torch.autograd.grad(out, leaves, grad_out)
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+def test_checkpoint_whose_first_saved_tensor_is_the_attentions(entry):
+    lin = torch.nn.Linear(64, 3 * 2 * 32, device="cuda", dtype=torch.float16)
+
+    def block(x):
+        qkv = lin(x).view(x.shape[0], x.shape[1], 3, 2, 32)
+        return _call(entry, [qkv] if entry == "packed" else qkv.permute(2, 0, 3, 1, 4).unbind(0), None)
+
+    x = torch.randn(2, 100, 64, device="cuda", dtype=torch.float16, requires_grad=True)
+    want = block(x)
+    grad_out = torch.randn_like(want)
+    want = torch.autograd.grad(want, [x, lin.weight, lin.bias], grad_out)
+    got = torch.autograd.grad(torch.utils.checkpoint.checkpoint(block, x, use_reentrant=False), [x, lin.weight, lin.bias], grad_out)
+    _assert_same(got, want)
