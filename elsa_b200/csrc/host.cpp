@@ -102,7 +102,8 @@ bool plain(const at::Tensor& t) {
   constexpr c10::DispatchKeySet special({c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::FuncTorchBatched,
                                          c10::DispatchKey::FuncTorchVmapMode, c10::DispatchKey::Python,
                                          c10::DispatchKey::Functionalize, c10::DispatchKey::Batched});
-  return t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has_any(special);
+  // (a forward-mode tangent too: the autograd functions of the general path refuse it, a result without one would be wrong)
+  return t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has_any(special) && !t._fw_grad(/*level=*/0).defined();
 }
 
 bool modes_active() { return c10::impl::TorchDispatchModeTLS::any_modes_set(); }

@@ -97,3 +97,17 @@ def test_checkpoint_whose_first_saved_tensor_is_the_attentions(entry):
     want = torch.autograd.grad(want, [x, lin.weight, lin.bias], grad_out)
     got = torch.autograd.grad(torch.utils.checkpoint.checkpoint(block, x, use_reentrant=False), [x, lin.weight, lin.bias], grad_out)
     _assert_same(got, want)
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("which", ["first", "last", "bias"])
+def test_forward_mode_is_refused_not_dropped(entry, which):
+    inputs, bias, _ = _problem(entry)
+    with torch.autograd.forward_ad.dual_level():
+        if which == "bias":
+            bias = torch.autograd.forward_ad.make_dual(bias, torch.ones_like(bias))
+        else:
+            i = 0 if which == "first" else -1
+            inputs[i] = torch.autograd.forward_ad.make_dual(inputs[i], torch.ones_like(inputs[i]))
+        with pytest.raises(NotImplementedError):
+            _call(entry, inputs, bias)
