@@ -14,6 +14,7 @@
 #include <torch/csrc/python_headers.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -106,7 +107,9 @@ bool plain(const at::Tensor& t) {
   return t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has_any(special) && !t._fw_grad(/*level=*/0).defined();
 }
 
-bool modes_active() { return c10::impl::TorchDispatchModeTLS::any_modes_set(); }
+// dispatch modes, and torch.jit.trace: the general path's autograd functions are recorded as operations of the graph, while
+// the output of a native call would be recorded as a constant
+bool modes_active() { return c10::impl::TorchDispatchModeTLS::any_modes_set() || at::tracer::impl::is_dispatch_enabled(); }
 
 struct Bias {
   at::Tensor t;               // fp32 contiguous [B|1, H|1, N, N]

@@ -111,3 +111,15 @@ def test_forward_mode_is_refused_not_dropped(entry, which):
             inputs[i] = torch.autograd.forward_ad.make_dual(inputs[i], torch.ones_like(inputs[i]))
         with pytest.raises(NotImplementedError):
             _call(entry, inputs, bias)
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("grad", [False, True])
+def test_a_traced_training_call_follows_its_inputs(entry, grad):
+    inputs, _, _ = _problem(entry, bias=False)
+    if grad:
+        inputs, _ = _leaves(inputs, None)
+    with torch.set_grad_enabled(grad):
+        traced = torch.jit.trace(lambda *x: _call(entry, x, None), tuple(inputs), check_trace=False)
+        other = [t * 0.5 + 0.1 for t in inputs]
+        _assert_same([traced(*other)], [_call(entry, other, None)])
