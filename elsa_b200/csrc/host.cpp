@@ -125,6 +125,8 @@ void bias_strides(Bias* b) {
   b->sk = st[3];
 }
 
+// Called with autograd in force where the result is saved: the detached tensor then shares the version counter of the
+// caller's, and a change of the bias between forward and backward is found.
 bool canonical_bias(const at::Tensor& bias, const Call& c, c10::Device dev, Bias* out) {
   if (!bias.defined()) return true;
   const int64_t dim = bias.dim();
@@ -244,9 +246,11 @@ void check_unpacked(const at::Tensor& t, at::IntArrayRef sizes, at::ScalarType d
 struct AttentionBackward : public torch::autograd::Node {
   Call c{};
   bool packed = false, bias_grad = false;
-  at::ScalarType dtype = at::kFloat, bias_dtype = at::kFloat;
-  std::vector<int64_t> bias_sizes, bias_shape;      // of the caller's bias and of the canonical one
-  SavedVariable q_, k_, v_, out_, state_, bias_;    // packed: q_ is the packed tensor, k_ and v_ stay empty
+  at::ScalarType dtype = at::kFloat, bias_dtype = at::kFloat, saved_bias_dtype = at::kFloat;
+  std::vector<int64_t> bias_sizes, saved_bias_sizes;
+  // packed: q_ is the packed tensor, k_ and v_ stay empty, bias_ is the canonical bias; else bias_ is the caller's (a 16-bit
+  // or expanded bias is kept as it is, and converted again by the backward)
+  SavedVariable q_, k_, v_, out_, state_, bias_;
 
   std::string name() const override { return packed ? "TwopassAttentionQkvpackedBackward" : "TwopassAttentionBackward"; }
 
@@ -279,9 +283,8 @@ struct AttentionBackward : public torch::autograd::Node {
     const at::Tensor state = aligned(s.state);
     Bias bias;
     if (s.bias.defined()) {
-      check_unpacked(s.bias, bias_shape, at::kFloat, dev);
-      bias.t = s.bias.contiguous();
-      bias_strides(&bias);
+      check_unpacked(s.bias, saved_bias_sizes, saved_bias_dtype, dev);
+      canonical_bias(s.bias, c, dev, &bias);
     }
     if (go.scalar_type() != dtype) go = go.to(dtype);
     c10::cuda::CUDAGuard guard(dev);
@@ -338,17 +341,20 @@ bool fill_call(Call* c, const at::Tensor& q, int64_t b, int64_t h, int64_t n, in
 }
 
 template <typename... V>
-std::shared_ptr<AttentionBackward> new_node(const Call& c, const at::Tensor& bias, const Bias& canon, const V&... inputs) {
+std::shared_ptr<AttentionBackward> new_node(const Call& c, bool packed, const at::Tensor& bias, const Bias& canon, const V&... inputs) {
   std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
   node->set_next_edges(torch::autograd::collect_next_edges(inputs..., bias));
   node->c = c;
+  node->packed = packed;
   node->dtype = c.dt == ELSA_F32 ? at::kFloat : c.dt == ELSA_F16 ? at::kHalf : at::kBFloat16;
   if (bias.defined()) {
+    const at::Tensor& saved = packed ? canon.t : bias;
     node->bias_grad = bias.requires_grad();
     node->bias_dtype = bias.scalar_type();
     node->bias_sizes = bias.sizes().vec();
-    node->bias_shape = canon.t.sizes().vec();
-    node->bias_ = SavedVariable(canon.t, false);
+    node->saved_bias_dtype = saved.scalar_type();
+    node->saved_bias_sizes = saved.sizes().vec();
+    node->bias_ = SavedVariable(saved, false);
   }
   return node;
 }
@@ -362,11 +368,11 @@ at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
   const bool record = train && at::GradMode::is_enabled() &&
                       (q.requires_grad() || k.requires_grad() || v.requires_grad() || (bias.defined() && bias.requires_grad()));
   Bias canon;
+  if (!canonical_bias(bias, c, q.device(), &canon)) return {};
   std::array<at::Tensor, 3> in{q, k, v};
   at::Tensor out, state;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    if (!canonical_bias(bias, c, q.device(), &canon)) return {};
     View t[3], o;
     const bool strided = pick_layouts(in, t);
     out = strided ? new_like_layout(in[0], t[0]) : new_tensor(q.sizes(), q, q.scalar_type());
@@ -375,7 +381,7 @@ at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
     run_forward(t, o, strided, canon, state, c, q.device());
   }
   if (record) {
-    auto node = new_node(c, bias, canon, q, k, v);
+    auto node = new_node(c, false, bias, canon, q, k, v);
     node->q_ = SavedVariable(in[0], false);
     node->k_ = SavedVariable(in[1], false);
     node->v_ = SavedVariable(in[2], false);
@@ -393,10 +399,10 @@ at::Tensor attention_packed(const at::Tensor& qkv, const at::Tensor& bias, Call 
     return {};
   const bool record = train && at::GradMode::is_enabled() && (qkv.requires_grad() || (bias.defined() && bias.requires_grad()));
   Bias canon;
+  if (!canonical_bias(bias, c, qkv.device(), &canon)) return {};
   at::Tensor out, state;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    if (!canonical_bias(bias, c, qkv.device(), &canon)) return {};
     out = new_bnhd(qkv, c.batch, c.heads, c.n, c.d);
     View in[3], o;
     packed_views(data_of(qkv), c, qkv.element_size(), in);
@@ -405,8 +411,7 @@ at::Tensor attention_packed(const at::Tensor& qkv, const at::Tensor& bias, Call 
     run_forward(in, o, true, canon, state, c, qkv.device());
   }
   if (record) {
-    auto node = new_node(c, bias, canon, qkv);
-    node->packed = true;
+    auto node = new_node(c, true, bias, canon, qkv);
     node->q_ = SavedVariable(qkv, false);
     node->state_ = SavedVariable(state, false);
     torch::autograd::set_history(out, node);

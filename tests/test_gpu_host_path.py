@@ -123,3 +123,44 @@ def test_a_traced_training_call_follows_its_inputs(entry, grad):
         traced = torch.jit.trace(lambda *x: _call(entry, x, None), tuple(inputs), check_trace=False)
         other = [t * 0.5 + 0.1 for t in inputs]
         _assert_same([traced(*other)], [_call(entry, other, None)])
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("form", ["leaf", "matrix", "heads", "batch"])
+def test_a_bias_changed_before_the_backward_is_found(entry, form):
+    inputs, bias, grad_out = _problem(entry)
+    inputs, leaf = _leaves(inputs, bias)
+    with torch.no_grad():
+        bias = {"leaf": leaf, "matrix": leaf[0], "heads": leaf, "batch": leaf[None]}[form]
+    out = _call(entry, inputs, bias if form == "leaf" else bias.detach())
+    with torch.no_grad():
+        leaf.add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(out, inputs, grad_out)
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("which", ["input", "out"])
+def test_an_input_or_output_changed_before_the_backward_is_found(entry, which):
+    inputs, bias, grad_out = _problem(entry)
+    inputs, bias = _leaves(inputs, bias)
+    out = _call(entry, inputs, bias)
+    with pytest.raises(RuntimeError):
+        with torch.no_grad():
+            (inputs[-1] if which == "input" else out).mul_(2)
+        torch.autograd.grad(out, inputs, grad_out)
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("form", ["heads", "expanded", "transposed"])
+def test_a_bias_alone_may_require_a_gradient(entry, dtype, form):
+    inputs, bias, grad_out = _problem(entry)
+    bias = bias.to(dtype)
+    if form == "transposed":
+        bias = bias.mT
+    leaf = bias.detach().requires_grad_(True)
+    used = leaf[None].expand(2, -1, -1, -1) if form == "expanded" else leaf
+    got, = torch.autograd.grad(_call(entry, inputs, used), leaf, grad_out)
+    want = _gradients(entry, inputs, bias.contiguous().float(), grad_out)[-1].to(dtype)
+    _assert_same([got], [want])
