@@ -25,6 +25,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 
 #include "../../include/elsa_b200.h"
 
@@ -243,33 +244,40 @@ void check_unpacked(const at::Tensor& t, at::IntArrayRef sizes, at::ScalarType d
               "a saved tensor of the attention came back from its unpack hook with another shape, dtype or device");
 }
 
-struct AttentionBackward : public torch::autograd::Node {
+// what a backward needs beside the saved tensors
+struct BackwardPlan {
   Call c{};
   bool packed = false, bias_grad = false;
   at::ScalarType dtype = at::kFloat, bias_dtype = at::kFloat, saved_bias_dtype = at::kFloat;
   std::vector<int64_t> bias_sizes, saved_bias_sizes;
-  // packed: q_ is the packed tensor, k_ and v_ stay empty, bias_ is the canonical bias; else bias_ is the caller's (a 16-bit
-  // or expanded bias is kept as it is, and converted again by the backward)
-  SavedVariable q_, k_, v_, out_, state_, bias_;
 
-  std::string name() const override { return packed ? "TwopassAttentionQkvpackedBackward" : "TwopassAttentionBackward"; }
-
-  void release_variables() override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    for (SavedVariable* s : {&q_, &k_, &v_, &out_, &state_, &bias_}) s->reset_data();
+  // the same as plain numbers and back, for compiled autograd
+  std::vector<int64_t> numbers() const {
+    std::vector<int64_t> x{c.batch, c.heads, c.n, c.d, c.dt, c.sdt, c.causal, c.part_width, c.q_chunk, packed, bias_grad,
+                           static_cast<int64_t>(dtype), static_cast<int64_t>(bias_dtype), static_cast<int64_t>(saved_bias_dtype)};
+    for (const auto* sizes : {&bias_sizes, &saved_bias_sizes}) {
+      x.push_back(static_cast<int64_t>(sizes->size()));
+      x.insert(x.end(), sizes->begin(), sizes->end());
+    }
+    return x;
+  }
+  static BackwardPlan of_numbers(const std::vector<int64_t>& x) {
+    BackwardPlan p;
+    size_t i = 0;
+    for (int* f : {&p.c.batch, &p.c.heads, &p.c.n, &p.c.d, &p.c.dt, &p.c.sdt, &p.c.causal, &p.c.part_width, &p.c.q_chunk}) *f = static_cast<int>(x.at(i++));
+    p.packed = x.at(i++) != 0;
+    p.bias_grad = x.at(i++) != 0;
+    for (at::ScalarType* f : {&p.dtype, &p.bias_dtype, &p.saved_bias_dtype}) *f = static_cast<at::ScalarType>(x.at(i++));
+    for (auto* sizes : {&p.bias_sizes, &p.saved_bias_sizes}) {
+      sizes->resize(x.at(i++));
+      for (int64_t& n : *sizes) n = x.at(i++);
+    }
+    return p;
   }
 
-  struct Saved { at::Tensor q, k, v, out, state, bias; };   // packed: q is the packed tensor
-
-  variable_list apply(variable_list&& grads) override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    if (!grads[0].defined()) return variable_list(packed ? 2 : 4);
-    // Unpacking runs the user's hooks, with autograd in force: a checkpoint repeats the forward in there, and the repeated
-    // forward has to record and save what the first one did.
-    Saved s{q_.unpack(), k_.unpack(), v_.unpack(), out_.unpack(shared_from_this()), state_.unpack(), bias_.unpack()};
-    at::AutoDispatchBelowADInplaceOrView below;
-    return gradients(std::move(s), std::move(grads[0]));
-  }
+  // packed: q is the packed tensor, k and v stay undefined, bias is the canonical bias; else bias is the caller's (a 16-bit or
+  // expanded bias is kept as it is, and converted again by the backward)
+  struct Saved { at::Tensor q, k, v, out, state, bias; };
 
   variable_list gradients(Saved s, at::Tensor go) const {
     variable_list result(packed ? 2 : 4);
@@ -329,6 +337,74 @@ struct AttentionBackward : public torch::autograd::Node {
   }
 };
 
+struct AttentionBackward : public torch::autograd::Node {
+  BackwardPlan plan;
+  SavedVariable q_, k_, v_, out_, state_, bias_;    // see BackwardPlan::Saved
+
+  std::string name() const override { return plan.packed ? "TwopassAttentionQkvpackedBackward" : "TwopassAttentionBackward"; }
+
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (SavedVariable* s : {&q_, &k_, &v_, &out_, &state_, &bias_}) s->reset_data();
+  }
+
+  BackwardPlan::Saved unpack() {
+    return {q_.unpack(), k_.unpack(), v_.unpack(), out_.unpack(shared_from_this()), state_.unpack(), bias_.unpack()};
+  }
+
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    if (!grads[0].defined()) return variable_list(plan.packed ? 2 : 4);
+    // Unpacking runs the user's hooks, with autograd in force: a checkpoint repeats the forward in there, and the repeated
+    // forward has to record and save what the first one did.
+    BackwardPlan::Saved s = unpack();
+    at::AutoDispatchBelowADInplaceOrView below;
+    return plan.gradients(std::move(s), std::move(grads[0]));
+  }
+
+  // Compiled autograd: the node is one opaque call of its graph, on the saved tensors and the plan.
+  void compiled_args(torch::dynamo::autograd::CompiledNodeArgs& args) const override {
+    args.collect(plan.numbers());
+    for (const SavedVariable* s : {&q_, &k_, &v_, &state_, &bias_}) args.collect(*s, false);
+    args.collect(out_, true);
+  }
+
+  variable_list apply_with_saved(const variable_list& grads, torch::dynamo::autograd::SwapSavedVariables& saved) override {
+    SavedVariable* const all[] = {&q_, &k_, &v_, &state_, &bias_, &out_};
+    for (SavedVariable* s : all) saved.before(*s);
+    BackwardPlan::Saved s = unpack();
+    torch::dynamo::autograd::PackedArgs packed;
+    std::vector<at::TypePtr> schema;
+    auto add = [&](const auto& x) {
+      packed.pack(x);
+      schema.emplace_back(torch::dynamo::autograd::IValuePacker<std::decay_t<decltype(x)>>::packed_type());
+    };
+    add(plan.numbers());
+    for (const at::Tensor* t : {&s.q, &s.k, &s.v, &s.out, &s.state, &s.bias}) add(*t);
+    const auto& compiler = torch::dynamo::autograd::getPyCompilerInterface();
+    const std::string fn = compiler->bind_function(saved.get_py_compiler(), name(), &call_packed, schema, /*is_custom_function=*/true, /*is_traceable=*/false);
+    variable_list result = compiler->call_function(saved.get_py_compiler(), "apply_functional", fn, grads, packed.vec(), output_metadata());
+    for (SavedVariable* s : all) saved.after(*s);
+    return result;
+  }
+
+  static variable_list call_packed(const variable_list& grads, const std::vector<c10::IValue>& values) {
+    torch::dynamo::autograd::PackedArgs packed(values);
+    const BackwardPlan plan = BackwardPlan::of_numbers(packed.unpack<std::vector<int64_t>>());
+    BackwardPlan::Saved s;
+    for (at::Tensor* t : {&s.q, &s.k, &s.v, &s.out, &s.state, &s.bias}) *t = packed.unpack<at::Tensor>();
+    if (!grads[0].defined()) return variable_list(plan.packed ? 2 : 4);
+    at::AutoDispatchBelowADInplaceOrView below;
+    return plan.gradients(std::move(s), grads[0]);
+  }
+
+  // shape, type and device of every input of the forward that gets a gradient
+  c10::IValue output_metadata() const {
+    return torch::dynamo::autograd::IValuePacker<std::vector<std::optional<torch::autograd::InputMetadata>>>::pack(
+        torch::dynamo::autograd::get_input_metadata(next_edges()));
+  }
+};
+
 bool fill_call(Call* c, const at::Tensor& q, int64_t b, int64_t h, int64_t n, int64_t d) {
   c->dt = dtype_code(q.scalar_type());
   if (c->dt < 0 || b <= 0 || h <= 0 || n <= 0 || d <= 0 || d > 128 || b > 65535 || h > 65535 || b * h > 65535 || n >= (1 << 30)) return false;
@@ -344,16 +420,17 @@ template <typename... V>
 std::shared_ptr<AttentionBackward> new_node(const Call& c, bool packed, const at::Tensor& bias, const Bias& canon, const V&... inputs) {
   std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
   node->set_next_edges(torch::autograd::collect_next_edges(inputs..., bias));
-  node->c = c;
-  node->packed = packed;
-  node->dtype = c.dt == ELSA_F32 ? at::kFloat : c.dt == ELSA_F16 ? at::kHalf : at::kBFloat16;
+  BackwardPlan& p = node->plan;
+  p.c = c;
+  p.packed = packed;
+  p.dtype = c.dt == ELSA_F32 ? at::kFloat : c.dt == ELSA_F16 ? at::kHalf : at::kBFloat16;
   if (bias.defined()) {
     const at::Tensor& saved = packed ? canon.t : bias;
-    node->bias_grad = bias.requires_grad();
-    node->bias_dtype = bias.scalar_type();
-    node->bias_sizes = bias.sizes().vec();
-    node->saved_bias_dtype = saved.scalar_type();
-    node->saved_bias_sizes = saved.sizes().vec();
+    p.bias_grad = bias.requires_grad();
+    p.bias_dtype = bias.scalar_type();
+    p.bias_sizes = bias.sizes().vec();
+    p.saved_bias_dtype = saved.scalar_type();
+    p.saved_bias_sizes = saved.sizes().vec();
     node->bias_ = SavedVariable(saved, false);
   }
   return node;

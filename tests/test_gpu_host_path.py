@@ -164,3 +164,18 @@ def test_a_bias_alone_may_require_a_gradient(entry, dtype, form):
     got, = torch.autograd.grad(_call(entry, inputs, used), leaf, grad_out)
     want = _gradients(entry, inputs, bias.contiguous().float(), grad_out)[-1].to(dtype)
     _assert_same([got], [want])
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("with_bias", [False, True])
+def test_backward_under_compiled_autograd(entry, with_bias):
+    from torch._dynamo import compiled_autograd
+    for n in (130, 70):
+        inputs, bias, grad_out = _problem(entry, n, bias=with_bias)
+        want = _gradients(entry, inputs, bias, grad_out)
+        for _ in range(2):
+            leaves, b = _leaves(inputs, bias)
+            out = _call(entry, leaves, b)
+            with compiled_autograd._enable(torch.compile(backend="eager")):
+                (out * 2).backward(grad_out / 2)
+            _assert_same([t.grad for t in leaves + ([b] if with_bias else [])], want)
