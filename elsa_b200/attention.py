@@ -94,12 +94,17 @@ def _check_qkv(q, k, v, who: str):
 def _resolve_keywords(*, block_m=None, block_n=None, q_chunk_size=None, summary_dtype=None, phase1_warps=None, phase2_warps=None,
                       phase1_stages=None, phase2_stages=None, input_precision="auto", algorithm="auto"):
     """The operator's keywords as the native host path takes them: (summary dtype code or -1 for the input's, partition
-    width, query chunk), after the same checks."""
-    sdt, part_width, q_chunk = _resolve_common(
-        None, algorithm=algorithm, input_precision=input_precision, summary_dtype=summary_dtype, block_m=block_m, block_n=block_n,
-        q_chunk_size=q_chunk_size, phase1_warps=phase1_warps, phase2_warps=phase2_warps, phase1_stages=phase1_stages,
-        phase2_stages=phase2_stages)
-    return -1 if sdt is None else _lib.dtype_code(sdt), part_width, q_chunk
+    width, query chunk).  None when a check fails: the general path then reports it, after the checks that come first there
+    (an empty sequence, for one, is answered before most keywords are looked at)."""
+    try:
+        sdt, part_width, q_chunk = _resolve_common(
+            None, algorithm=algorithm, input_precision=input_precision, summary_dtype=summary_dtype, block_m=block_m,
+            block_n=block_n, q_chunk_size=q_chunk_size, phase1_warps=phase1_warps, phase2_warps=phase2_warps,
+            phase1_stages=phase1_stages, phase2_stages=phase2_stages)
+    except (TypeError, ValueError, OverflowError):
+        return None
+    # (wider than any sequence is one partition, or one chunk)
+    return -1 if sdt is None else _lib.dtype_code(sdt), min(part_width, 1 << 30), min(q_chunk, 1 << 30)
 
 
 def _resolve_common(q, *, algorithm, input_precision, summary_dtype, block_m, block_n, q_chunk_size,
@@ -286,13 +291,14 @@ def twopass_attention(
     would run them (fp16, D = 64, no bias, not causal); by default the scale is applied exactly, in fp32.
     """
     if not reference_rounding and isinstance(q, torch.Tensor) and q.is_cuda:
-        sdt, part_width, q_chunk = _resolve_keywords(
+        keywords = _resolve_keywords(
             block_m=block_m, block_n=block_n, q_chunk_size=q_chunk_size, summary_dtype=summary_dtype, phase1_warps=phase1_warps,
             phase2_warps=phase2_warps, phase1_stages=phase1_stages, phase2_stages=phase2_stages, input_precision=input_precision,
             algorithm=algorithm)
-        out = _lib.host().attention(q, k, v, bias, is_causal, sdt, part_width, q_chunk, False)
-        if out is not None:
-            return out
+        if keywords is not None:
+            out = _lib.host().attention(q, k, v, bias, is_causal, *keywords, False)
+            if out is not None:
+                return out
     # the general path: what the native one does not cover, and the errors
     _check_qkv(q, k, v, "twopass_attention")
     if algorithm not in ("auto", "paper_scan"):

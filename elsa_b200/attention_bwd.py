@@ -196,12 +196,17 @@ def twopass_attention_backward(
     return dq, dk, dv
 
 
+_KEYWORDS = frozenset(_resolve_keywords.__kwdefaults__)
+
+
 def _native_keywords(fwd_kwargs: dict):
-    """(summary dtype code, partition width, query chunk) for the native host path."""
+    """(summary dtype code, partition width, query chunk) for the native host path, or None: see `_resolve_keywords`."""
     if not fwd_kwargs:
         return -1, 0, 0
     if "reference_rounding" in fwd_kwargs:
         fwd_kwargs = {name: val for name, val in fwd_kwargs.items() if name != "reference_rounding"}
+    if not _KEYWORDS.issuperset(fwd_kwargs):
+        return None
     return _resolve_keywords(**fwd_kwargs)
 
 
@@ -431,9 +436,11 @@ def twopass_attention_qkvpacked(qkv: torch.Tensor, *, bias: Optional[torch.Tenso
     if fwd_kwargs:
         fwd_kwargs = {name: val for name, val in fwd_kwargs.items() if not name.startswith("bwd_")}
     if qkv.is_cuda and not fwd_kwargs.get("reference_rounding", False):
-        out = _lib.host().attention_packed(qkv, bias, is_causal, *_native_keywords(fwd_kwargs), bool(train))
-        if out is not None:
-            return out
+        keywords = _native_keywords(fwd_kwargs)
+        if keywords is not None:
+            out = _lib.host().attention_packed(qkv, bias, is_causal, *keywords, bool(train))
+            if out is not None:
+                return out
     # the general path: what the native one does not cover, and the errors
     if not train:
         if not fwd_kwargs.get("reference_rounding", False) and _packed_fast_ok(qkv):
@@ -469,9 +476,11 @@ def twopass_attention_train(
     if bwd_num_warps is not None:
         _validate_warps("num_warps", bwd_num_warps)
     if isinstance(q, torch.Tensor) and q.is_cuda and not fwd_kwargs.get("reference_rounding", False):
-        out = _lib.host().attention(q, k, v, bias, is_causal, *_native_keywords(fwd_kwargs), True)
-        if out is not None:
-            return out
+        keywords = _native_keywords(fwd_kwargs)
+        if keywords is not None:
+            out = _lib.host().attention(q, k, v, bias, is_causal, *keywords, True)
+            if out is not None:
+                return out
     # the general path: what the native one does not cover, and the errors
     bwd_kwargs = {name: val for name, val in (("block_m", bwd_block_m), ("block_n", bwd_block_n),
                                               ("num_warps", bwd_num_warps), ("num_stages", bwd_num_stages))

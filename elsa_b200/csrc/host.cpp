@@ -512,8 +512,8 @@ bool get_call(PyObject* const* a, Call* c) {          // causal, summary dtype c
   if (causal < 0) return false;
   c->causal = causal;
   c->sdt = static_cast<int>(PyLong_AsLong(a[1]));
-  c->part_width = static_cast<int>(std::min<long>(PyLong_AsLong(a[2]), 1 << 30));
-  c->q_chunk = static_cast<int>(std::min<long>(PyLong_AsLong(a[3]), 1 << 30));
+  c->part_width = static_cast<int>(PyLong_AsLong(a[2]));
+  c->q_chunk = static_cast<int>(PyLong_AsLong(a[3]));
   return !PyErr_Occurred();
 }
 

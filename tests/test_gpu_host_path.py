@@ -179,3 +179,26 @@ def test_backward_under_compiled_autograd(entry, with_bias):
             with compiled_autograd._enable(torch.compile(backend="eager")):
                 (out * 2).backward(grad_out / 2)
             _assert_same([t.grad for t in leaves + ([b] if with_bias else [])], want)
+
+
+def _infer(inputs, bias, **kwargs):
+    return E.twopass_attention(*inputs, bias=bias, **kwargs)
+
+
+@pytest.mark.parametrize("entry", ENTRIES + ["infer"])
+def test_keywords_are_checked_in_the_order_of_the_general_path(entry):
+    call = _infer if entry == "infer" else lambda *a, **kw: _call(entry, *a, **kw)
+    layout = "packed" if entry == "packed" else "op"
+    # an empty sequence is answered before the keywords are looked at
+    empty = [torch.empty((2, 0, 3, 3, 64) if entry == "packed" else (2, 3, 0, 64), device="cuda") for _ in range(1 if entry == "packed" else 3)]
+    assert call(empty, None, phase1_warps=3).shape == (2, 3, 0, 64)
+    inputs, _, _ = _problem(layout, bias=False)
+    with pytest.raises(ValueError, match="must have shape"):
+        call([t[0] for t in inputs], None, phase1_warps=3)
+    with pytest.raises(ValueError, match="phase1_warps"):
+        call(inputs, None, phase1_warps=3)
+    with pytest.raises(ValueError, match="algorithm"):
+        call(inputs, None, algorithm="other")
+    with pytest.raises(TypeError, match="nope"):
+        call(inputs, None, nope=1)
+    _assert_same([call(inputs, None, block_n=1 << 70, q_chunk_size=1 << 70)], [call(inputs, None)])
