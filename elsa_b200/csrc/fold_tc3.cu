@@ -26,9 +26,10 @@
 //                              fp32 additions
 //
 // Scales.  The plane scales of the q, k, v tiles are powers of two, so they come out exactly: the scores of a tile pair
-// arrive times s_q s_k (divided out together with the softmax scale), O of a key tile times s_v (divided out when it is
-// taken into the running sum), and P is produced times 2^14 by adding 14 to the exponent of the exponential (so the row
-// sum and the output carry 2^14 until the epilogue).
+// arrive times s_q s_k (divided out together with the softmax scale), P is produced times 2^14 by adding 14 to the exponent
+// of the exponential, and O of a key tile arrives times 2^14 s_v: both are divided out when it is taken into the running
+// sum, which so has the range of the result (2^14 left in it until the epilogue made |v| z >= 2^114 infinite).  The row sum
+// carries 2^14 until the epilogue.
 // With fp16 planes a weight must not exceed 1, so the reference max follows every key tile (no lazy rescale).
 //
 // The per-element work of the fold is about a dozen instructions; with one thread per row (four warps, one per
@@ -345,7 +346,7 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const float cq_scale = prm.scale_log2 * prm.inv_q[static_cast<int64_t>(bh) * ((prm.n_ctx + kPlaneRows - 1) / kPlaneRows) + min(q0, prm.n_ctx - 1) / kPlaneRows];
     const float* inv_k = prm.inv_k + static_cast<int64_t>(bh) * tiles_k + k_begin / kPlaneRows;
     const float* inv_v = prm.inv_v + static_cast<int64_t>(bh) * tiles_k + k_begin / kPlaneRows;
-    float ik_next = n_t > 0 ? inv_k[0] : 1.f, iv_next = n_t > 0 ? inv_v[0] : 1.f, iv = 1.f;   // iv: of the tile whose O is in flight
+    float ik_next = n_t > 0 ? inv_k[0] : 1.f, iv_next = n_t > 0 ? inv_v[0] : 1.f, iv = 1.f;   // iv: 1 / (2^14 s_v) of the tile whose O is in flight
     const float* bias_row = nullptr;
     if constexpr (BIAS) {
       const int bi = bh / prm.heads, hi = bh - bi * prm.heads;
@@ -457,7 +458,7 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         tc_fence_after();
         take_o();
       }
-      iv = iv_this;
+      iv = iv_this * kUnitInverse;
       if (move) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) o_run[i] *= alpha;
@@ -497,9 +498,8 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       if (alive) {
         const float ztot = (row_sum[0][row] + row_sum[1][row]) + (row_sum[2][row] + row_sum[3][row]);
-        // zsum and o_run carry kPlaneUnit (a power of two: taken out exactly)
-        const float f = (m_true == -CUDART_INF_F) ? 0.f : exp2f(m_ref - m_true - kLog2Unit);
-        z_out = ztot * f;
+        const float f = (m_true == -CUDART_INF_F) ? 0.f : exp2f(m_ref - m_true);
+        z_out = ztot * kUnitInverse * f;       // (powers of two: taken out exactly)
         m_out = z_out > 0.f ? m_true : -CUDART_INF_F;
 #pragma unroll
         for (int i = 0; i < 16; ++i) o_run[i] = z_out > 0.f ? o_run[i] * f : 0.f;

@@ -326,6 +326,7 @@ __device__ __forceinline__ void st_global_v8(float* p, const float (&r)[8]) {
 constexpr int kPlanes = ELSA_FP32_PLANES;
 static_assert(kPlanes == 2 || kPlanes == 3, "fp32 operands are split into two fp16 or three bf16 planes");
 constexpr float kLog2Unit = kPlanes == 2 ? 14.f : 0.f;        // log2 of what a probability (<= 1) is multiplied by before its split
+constexpr float kUnitInverse = kPlanes == 2 ? 1.f / 16384.f : 1.f;
 constexpr int kPlaneRows = 128;                                // rows that share one scale
 constexpr uint32_t kPlaneFmt = kPlanes == 3 ? 1u : 0u;         // tcgen05 operand format: bf16 / fp16
 constexpr int kPlaneDtype = kPlanes == 3 ? ELSA_BF16 : ELSA_F16;

@@ -386,3 +386,18 @@ def test_default_plan_of_the_tensor_core_fold():
     assert parts(2, 1, 8, 16384, 64, 1) == 2
     assert parts(1, 1, 8, 8192, 64, 0) == 1 and parts(1, 1, 8, 8192, 64, 1) == 2
     assert parts(1, 64, 3, 197, 64, 0) == 1
+
+
+@pytest.mark.parametrize("mag", [8e30, 1e-36])
+@pytest.mark.parametrize("n,block_n", [(8192, 8192), (4097, 1024)])
+@pytest.mark.parametrize("biased", [False, True])
+def test_fp32_tensor_core_fold_keeps_the_range_of_the_result(mag, n, block_n, biased):
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    q, k = (0.01 * torch.randn((1, 2, n, 64), generator=gen, device="cuda") for _ in range(2))
+    v = mag * (0.5 + 0.5 * torch.rand((1, 2, n, 64), generator=gen, device="cuda"))   # one sign: the running sum reaches n |v|
+    bias = 0.01 * torch.randn((1, 1, n, n), generator=gen, device="cuda") if biased else None
+    out = E.twopass_attention(q, k, v, bias=bias, block_n=block_n).double() / mag
+    s = q.double() @ k.double().mT / 8
+    ref = torch.softmax(s if bias is None else s + bias, -1) @ (v.double() / mag)
+    # 1e-36 is below the smallest plane scale (2^-100): its planes keep 22 - 7 bits fewer of the small side, 4e-6 relative
+    assert (out - ref).norm() <= (1e-6 if mag > 1 else 4e-6) * ref.norm()
