@@ -1,12 +1,14 @@
 """ctypes binding of libelsa_b200.so (the C ABI declared in include/elsa_b200.h).
 
 The library is built ahead of time by `python -m elsa_b200.build` (or `__graft_entry__.build()`)
-and lives next to this file.  There is no fallback: if it is missing, every operator raises.
+and lives next to this file.  There is no fallback: if it is missing, every operator raises.  (The host
+path next to it, _host.so, only shortens the way to the library: see `host`.)
 """
 from __future__ import annotations
 
 import ctypes
 import os
+import warnings
 from ctypes import c_char_p, c_int, c_int64, c_uint, c_uint64, c_void_p, POINTER
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -86,20 +88,33 @@ _HOST_ENTRIES = ("elsa_forward_workspace_bytes", "elsa_twopass_forward", "elsa_t
                  "elsa_backward_workspace_bytes", "elsa_twopass_backward", "elsa_twopass_backward_strided", "elsa_strerror",
                  "elsa_last_cuda_error")
 _host_module = None
+_host_tried = False
+
+
+def _load_host():
+    import torch
+    lib = load()
+    try:
+        from . import _host as mod
+    except ImportError as exc:
+        why = f"does not load ({exc})"
+    else:
+        if mod.torch_version == torch.__version__:
+            mod.bind({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in _HOST_ENTRIES})
+            return mod
+        why = f"was built for torch {mod.torch_version}, this is {torch.__version__}"
+    warnings.warn(f"elsa_b200/_host.so {why}: operators take their general path, with the same kernels and more host time per "
+                  "call; build it with `python -m elsa_b200.build`", RuntimeWarning, stacklevel=4)
+    return None
 
 
 def host():
-    """The native host path (csrc/host.cpp), bound to the loaded library; raises RuntimeError when it has not been built."""
-    global _host_module
-    if _host_module is None:
-        lib = load()
-        try:
-            from . import _host as mod
-        except ImportError as exc:
-            raise RuntimeError(f"elsa_b200/_host.so is missing or does not load ({exc}): build it with "
-                               "`python -m elsa_b200.build`") from exc
-        mod.bind({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in _HOST_ENTRIES})
-        _host_module = mod
+    """The native host path (csrc/host.cpp), bound to the loaded library; None, after one warning, where it has not been built
+    for this torch: it uses torch's C++ interface, which changes with the version."""
+    global _host_module, _host_tried
+    if not _host_tried:
+        _host_module = _load_host()
+        _host_tried = True
     return _host_module
 
 

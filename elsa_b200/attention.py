@@ -295,8 +295,9 @@ def twopass_attention(
             block_m=block_m, block_n=block_n, q_chunk_size=q_chunk_size, summary_dtype=summary_dtype, phase1_warps=phase1_warps,
             phase2_warps=phase2_warps, phase1_stages=phase1_stages, phase2_stages=phase2_stages, input_precision=input_precision,
             algorithm=algorithm)
-        if keywords is not None:
-            out = _lib.host().attention(q, k, v, bias, is_causal, *keywords, False)
+        host = _lib.host()
+        if keywords is not None and host is not None:
+            out = host.attention(q, k, v, bias, is_causal, *keywords, False)
             if out is not None:
                 return out
     # the general path: what the native one does not cover, and the errors

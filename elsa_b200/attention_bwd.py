@@ -436,9 +436,9 @@ def twopass_attention_qkvpacked(qkv: torch.Tensor, *, bias: Optional[torch.Tenso
     if fwd_kwargs:
         fwd_kwargs = {name: val for name, val in fwd_kwargs.items() if not name.startswith("bwd_")}
     if qkv.is_cuda and not fwd_kwargs.get("reference_rounding", False):
-        keywords = _native_keywords(fwd_kwargs)
-        if keywords is not None:
-            out = _lib.host().attention_packed(qkv, bias, is_causal, *keywords, bool(train))
+        host, keywords = _lib.host(), _native_keywords(fwd_kwargs)
+        if host is not None and keywords is not None:
+            out = host.attention_packed(qkv, bias, is_causal, *keywords, bool(train))
             if out is not None:
                 return out
     # the general path: what the native one does not cover, and the errors
@@ -476,9 +476,9 @@ def twopass_attention_train(
     if bwd_num_warps is not None:
         _validate_warps("num_warps", bwd_num_warps)
     if isinstance(q, torch.Tensor) and q.is_cuda and not fwd_kwargs.get("reference_rounding", False):
-        keywords = _native_keywords(fwd_kwargs)
-        if keywords is not None:
-            out = _lib.host().attention(q, k, v, bias, is_causal, *keywords, True)
+        host, keywords = _lib.host(), _native_keywords(fwd_kwargs)
+        if host is not None and keywords is not None:
+            out = host.attention(q, k, v, bias, is_causal, *keywords, True)
             if out is not None:
                 return out
     # the general path: what the native one does not cover, and the errors

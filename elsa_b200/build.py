@@ -17,6 +17,7 @@ OBJ_DIR = os.path.join(CSRC, "build")
 LIB_PATH = os.path.join(HERE, "libelsa_b200.so")
 HOST_SRC = os.path.join(CSRC, "host.cpp")
 HOST_PATH = os.path.join(HERE, "_host.so")
+HOST_STAMP = os.path.join(OBJ_DIR, "_host.built_for")
 SOURCES = ["api.cu", "phase2.cu", "fold_simt.cu", "bwd_simt.cu", "fold_tc.cu", "fold_tc3.cu", "fold_tcw.cu", "bwd_tc.cu", "bwd_tc3.cu", "bwd_tcw.cu", "win_tc.cu", "peaks.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -41,9 +42,20 @@ def needs_build() -> bool:
     return not os.path.exists(LIB_PATH) or os.path.getmtime(LIB_PATH) < _newest_source_mtime()
 
 
+def _host_built_for() -> str:
+    """What _host.so depends on beside its sources: torch's C++ interface and Python's."""
+    import sysconfig
+
+    import torch
+    return f"torch {torch.__version__} {sysconfig.get_config_var('SOABI')}"
+
+
 def host_needs_build() -> bool:
     newest = max(os.path.getmtime(HOST_SRC), os.path.getmtime(os.path.join(os.path.dirname(HERE), "include", "elsa_b200.h")))
-    return not os.path.exists(HOST_PATH) or os.path.getmtime(HOST_PATH) < newest
+    if not os.path.exists(HOST_PATH) or os.path.getmtime(HOST_PATH) < newest or not os.path.exists(HOST_STAMP):
+        return True
+    with open(HOST_STAMP) as f:
+        return f.read() != _host_built_for()
 
 
 def build_host() -> None:
@@ -56,12 +68,15 @@ def build_host() -> None:
                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     lib = os.path.join(root, "lib")
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{path}" for path in include), HOST_SRC,
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DELSA_TORCH_VERSION="{torch.__version__}"', *(f"-I{path}" for path in include), HOST_SRC,
            "-o", HOST_PATH, f"-L{lib}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10",
            f"-Wl,-rpath,{lib}"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed for host.cpp:\n{res.stdout}\n{res.stderr}")
+    os.makedirs(OBJ_DIR, exist_ok=True)
+    with open(HOST_STAMP, "w") as f:
+        f.write(_host_built_for())
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -587,4 +587,8 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, kMethods, nu
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m && PyModule_AddStringConstant(m, "torch_version", ELSA_TORCH_VERSION) < 0) Py_CLEAR(m);
+  return m;
+}

@@ -127,3 +127,34 @@ def test_packed_plan_strides_match_the_views():
     arr = tuple(plan.backward_strides(gs))
     assert arr[:9] == tuple(plan.qkv_strides) * 3 and arr[9:12] == tuple(plan.out_strides) and arr[12:15] == gs
     assert arr[15:] == tuple(plan.qkv_strides) * 3 and plan.fwd_ws >= 0 and plan.bwd_ws >= 0
+
+
+def test_host_path_is_rebuilt_for_another_torch(lib, monkeypatch, tmp_path):
+    from elsa_b200 import build
+    assert not build.host_needs_build()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert build.host_needs_build()
+    monkeypatch.undo()
+    monkeypatch.setattr(build, "HOST_STAMP", str(tmp_path / "absent"))
+    assert build.host_needs_build()
+
+
+@pytest.mark.parametrize("how", ["missing", "other torch", "built"])
+def test_host_path_that_does_not_fit_is_left_out(lib, monkeypatch, how):
+    import sys
+    import warnings
+
+    import elsa_b200
+    from elsa_b200 import _lib
+    monkeypatch.setattr(_lib, "_host_tried", False)
+    monkeypatch.setattr(_lib, "_host_module", None)
+    if how == "missing":
+        monkeypatch.setitem(sys.modules, "elsa_b200._host", None)
+        monkeypatch.delattr(elsa_b200, "_host", raising=False)
+    elif how == "other torch":
+        monkeypatch.setattr(torch, "__version__", "0.0.1")
+    with warnings.catch_warnings(record=True) as caught:
+        warnings.simplefilter("always")
+        first, second = _lib.host(), _lib.host()
+    assert (first is None) == (how != "built") and second is first
+    assert len(caught) == (0 if how == "built" else 1)

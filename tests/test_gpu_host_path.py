@@ -202,3 +202,15 @@ def test_keywords_are_checked_in_the_order_of_the_general_path(entry):
     with pytest.raises(TypeError, match="nope"):
         call(inputs, None, nope=1)
     _assert_same([call(inputs, None, block_n=1 << 70, q_chunk_size=1 << 70)], [call(inputs, None)])
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+def test_operators_work_without_the_host_path(entry, monkeypatch):
+    from elsa_b200 import _lib
+    inputs, bias, grad_out = _problem(entry)
+    want = [_call(entry, inputs, bias), *_gradients(entry, inputs, bias, grad_out)]
+    monkeypatch.setattr(_lib, "_host_module", None)
+    monkeypatch.setattr(_lib, "_host_tried", True)
+    _assert_same([_call(entry, inputs, bias), *_gradients(entry, inputs, bias, grad_out)], want)
+    if entry == "op":
+        _assert_same([_infer(inputs, bias)], want[:1])
