@@ -3,6 +3,7 @@ path of the Python operators (g++ against the headers of the installed torch).
 
     python -m elsa_b200.build            # build if sources are newer than the library
     python -m elsa_b200.build --force
+    python elsa_b200/build.py --library  # the C library alone: needs nvcc only, neither torch nor Python's headers
 """
 from __future__ import annotations
 
@@ -80,8 +81,14 @@ def build_host() -> None:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
+    """Both files, the C library first: it is there whatever becomes of the host path."""
+    path = build_library(force, verbose)
     if force or host_needs_build():
         build_host()
+    return path
+
+
+def build_library(force: bool = False, verbose: bool = False) -> str:
     if not force and not needs_build():
         return LIB_PATH
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -109,4 +116,5 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 if __name__ == "__main__":
-    print(build(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
+    make = build_library if "--library" in sys.argv else build
+    print(make(force="--force" in sys.argv, verbose="--verbose" in sys.argv))

@@ -158,3 +158,20 @@ def test_host_path_that_does_not_fit_is_left_out(lib, monkeypatch, how):
         first, second = _lib.host(), _lib.host()
     assert (first is None) == (how != "built") and second is first
     assert len(caught) == (0 if how == "built" else 1)
+
+
+def test_the_c_library_needs_no_torch_and_comes_first(lib, monkeypatch):
+    import subprocess
+    import sys
+
+    from elsa_b200 import build
+    done = []
+    monkeypatch.setattr(build, "build_library", lambda *a: done.append("library") or build.LIB_PATH)
+    monkeypatch.setattr(build, "build_host", lambda: done.append("host"))
+    build.build(force=True)
+    assert done == ["library", "host"]
+    # as a script, with neither torch nor the package importable
+    code = ("import sys, runpy; sys.modules['torch'] = sys.modules['elsa_b200'] = None; sys.argv = ['build.py', '--library']; "
+            f"runpy.run_path({build.__file__!r}, run_name='__main__')")
+    res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600)
+    assert res.returncode == 0 and res.stdout.strip() == build.LIB_PATH, res.stderr
