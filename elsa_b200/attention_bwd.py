@@ -65,6 +65,10 @@ def twopass_attention_with_state(
     return out, row_m, row_z
 
 
+def _repeatable_flag() -> int:
+    return _lib.FLAG_REPEATABLE if torch.are_deterministic_algorithms_enabled() else 0
+
+
 def _row_stats(q_c, k_c, meta, is_causal):
     lib = _lib.load()
     batch, heads, seq_len, head_dim = map(int, q_c.shape)
@@ -126,6 +130,7 @@ def _backward_impl(q, k, v, out, grad_out, *, bias, is_causal, row_m, row_z, wan
         # same broadcast layout as the bias itself: contributions of broadcast axes are summed
         dbias = torch.zeros_like(meta.tensor)
         dargs = (dbias.data_ptr(), meta.stride_b, meta.stride_h, meta.stride_q, meta.stride_k)
+    flags |= _repeatable_flag()
     dt = _lib.dtype_code(q.dtype)
     nbytes = _cached_bytes("elsa_backward_workspace_bytes", dt, batch, heads, seq_len, head_dim, int(meta.has_bias),
                            int(bool(is_causal)), flags)
@@ -384,7 +389,7 @@ class _PackedQkvAttentionAutograd(torch.autograd.Function):
                 base, base + step, base + 2 * step, out.data_ptr(), grad_out.data_ptr(), plan.backward_strides(gs),
                 state.data_ptr(), state.data_ptr() + 2 * state.numel(), *meta.c_args(),
                 dbase, dbase + step, dbase + 2 * step, *dargs, ws.data_ptr(), ws.numel(), plan.dt, batch, heads, seq_len,
-                head_dim, int(ctx.is_causal), 0, _lib.raw_stream(qkv.device))
+                head_dim, int(ctx.is_causal), _repeatable_flag(), _lib.raw_stream(qkv.device))
         _lib.check(rc, "elsa_twopass_backward")
         return dqkv, dbias
 

@@ -619,9 +619,9 @@ static int backward_impl(const void* q, const void* k, const void* v, const void
   float* row_d = reinterpret_cast<float*>(ws);
   float* row_lse = reinterpret_cast<float*>(ws + bwd_state_bytes(batch, heads, n_ctx));
   // d <= 64, 16-bit: the five-contraction kernel, for a biased problem only when its gradient is asked for.  It reads the bias
-  // and writes dbias once, where the two kernels of bwd_tcw.cu read the bias twice, but adds dQ in arrival order; without a
-  // bias gradient the biased backward keeps the order-independent kernels (its dq repeats bit for bit).
-  const bool use_tc = (bias == nullptr) == (dbias == nullptr) && tc_backward_ok(dtype, head_dim, n_ctx, batch * heads, bias != nullptr, flags);
+  // and writes dbias once, where the kernel of bwd_tcw.cu reads the bias twice, but adds dQ in arrival order; without a
+  // bias gradient, or on request, the biased backward keeps the order-independent kernel (its dq repeats bit for bit).
+  const bool use_tc = (bias == nullptr) == (dbias == nullptr) && !(bias && (flags & ELSA_FLAG_REPEATABLE)) && tc_backward_ok(dtype, head_dim, n_ctx, batch * heads, bias != nullptr, flags);
   const bool use_tc3 = (dbias == nullptr || bias != nullptr) && tc3_backward_ok(dtype, head_dim, n_ctx, batch * heads, bias != nullptr, flags);
   // (the wide-head kernels also take biased problems, with or without a bias gradient)
   const bool use_tcw = !use_tc && !use_tc3 && (dbias == nullptr || bias != nullptr) &&

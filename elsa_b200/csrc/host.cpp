@@ -170,7 +170,8 @@ void run_forward(const View (&in)[3], const View& out, bool strided, const Bias&
 // t: q, k, v, out, dout, dq, dk, dv
 void run_backward(const View (&t)[8], bool strided, const Bias& bias, const at::Tensor& dbias, const at::Tensor& state, const Call& c,
                   c10::Device dev) {
-  const int64_t need = f_bwd_ws(c.dt, c.batch, c.heads, c.n, c.d, bias.t.defined(), c.causal, 0u);
+  const unsigned flags = at::globalContext().deterministicAlgorithms() ? ELSA_FLAG_REPEATABLE : 0u;
+  const int64_t need = f_bwd_ws(c.dt, c.batch, c.heads, c.n, c.d, bias.t.defined(), c.causal, flags);
   TORCH_CHECK_VALUE(need >= 0, "elsa_b200: unsupported problem size for the backward");
   const int64_t bytes = std::max<int64_t>(need, 256);
   c10::DataPtr ws = workspace(bytes);
@@ -186,10 +187,10 @@ void run_backward(const View (&t)[8], bool strided, const Bias& bias, const at::
       for (int j = 0; j < 3; ++j) st[3 * i + j] = t[i].st[j];
     rc = f_bwd_strided(t[0].p, t[1].p, t[2].p, t[3].p, t[4].p, st, rm, rz, bias.ptr(), bias.sb, bias.sh, bias.sq, bias.sk, t[5].p,
                        t[6].p, t[7].p, db, ds[0], ds[1], ds[2], ds[3], ws.get(), bytes, c.dt, c.batch, c.heads, c.n, c.d,
-                       c.causal, 0u, stream);
+                       c.causal, flags, stream);
   } else {
     rc = f_bwd(t[0].p, t[1].p, t[2].p, t[3].p, t[4].p, rm, rz, bias.ptr(), bias.sb, bias.sh, bias.sq, bias.sk, t[5].p, t[6].p,
-               t[7].p, db, ds[0], ds[1], ds[2], ds[3], ws.get(), bytes, c.dt, c.batch, c.heads, c.n, c.d, c.causal, 0u, stream);
+               t[7].p, db, ds[0], ds[1], ds[2], ds[3], ws.get(), bytes, c.dt, c.batch, c.heads, c.n, c.d, c.causal, flags, stream);
   }
   check_status(rc, "elsa_twopass_backward");
 }

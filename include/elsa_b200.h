@@ -53,6 +53,8 @@ enum elsa_status {
                                      three cross products per fp32 product: the accuracy class of 3xTF32; the planes
                                      cost the size of q, k, v in forward workspace and of q, dout, k, v in backward
                                      workspace) */
+#define ELSA_FLAG_REPEATABLE 32u  /* backward, 16-bit inputs with a bias whose gradient is asked for, head dim <= 64: the kernels whose
+                                     dq repeats bit for bit from run to run, instead of the faster one that adds dq in arrival order */
 #define ELSA_FLAG_REF_ROUNDING 8u /* forward, fp16 / head dim 64 / no bias / not causal only: reproduce the rounding points of
                                      the reference's fp16 d=64 kernels (q * log2(e)/8 formed in fp16, scores unscaled:
                                      attention_parallel_scan.py:153-154,160) instead of the exact fp32 scale; the workspace

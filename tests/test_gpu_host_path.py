@@ -214,3 +214,38 @@ def test_operators_work_without_the_host_path(entry, monkeypatch):
     _assert_same([_call(entry, inputs, bias), *_gradients(entry, inputs, bias, grad_out)], want)
     if entry == "op":
         _assert_same([_infer(inputs, bias)], want[:1])
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("native", [True, False])
+def test_biased_gradients_repeat_when_torch_is_asked_for_it(entry, native, monkeypatch):
+    from elsa_b200 import _lib
+    if not native:
+        monkeypatch.setattr(_lib, "_host_module", None)
+        monkeypatch.setattr(_lib, "_host_tried", True)
+    inputs, bias, grad_out = _problem(entry, n=700, b=1)     # (b = 1: the bias gradient is not summed over anything)
+    loose = _gradients(entry, inputs, bias, grad_out)
+    torch.use_deterministic_algorithms(True)
+    try:
+        first, *rest = (_gradients(entry, inputs, bias, grad_out) for _ in range(6))
+    finally:
+        torch.use_deterministic_algorithms(False)
+    for again in rest:
+        assert all(torch.equal(a, b) for a, b in zip(first, again))
+    _assert_same(first, loose)
+
+
+@pytest.mark.parametrize("entry", ENTRIES)
+@pytest.mark.parametrize("n,dtype", [(49, torch.float16), (130, torch.bfloat16), (130, torch.float32)])
+def test_under_a_dispatch_mode_the_general_path_agrees(entry, n, dtype):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Passing(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    inputs, bias, grad_out = _problem(entry, n, dtype)
+    want = [_call(entry, inputs, bias), *_gradients(entry, inputs, bias, grad_out)]
+    with Passing():
+        got = [_call(entry, inputs, bias), *_gradients(entry, inputs, bias, grad_out)]
+    _assert_same(got, want)
