@@ -113,32 +113,24 @@ bool plain(const at::Tensor& t) {
 bool modes_active() { return c10::impl::TorchDispatchModeTLS::any_modes_set() || at::tracer::impl::is_dispatch_enabled(); }
 
 struct Bias {
-  at::Tensor t;               // fp32 contiguous [B|1, H|1, N, N]
+  at::Tensor t;               // fp32, contiguous: [B|1, H|1, N, N] up to leading axes of size 1
   int64_t sb = 0, sh = 0, sq = 0, sk = 0;
   const float* ptr() const { return t.defined() ? t.const_data_ptr<float>() : nullptr; }
 };
 
-void bias_strides(Bias* b) {
-  const auto st = b->t.strides();
-  b->sb = b->t.size(0) == 1 ? 0 : st[0];
-  b->sh = b->t.size(1) == 1 ? 0 : st[1];
-  b->sq = st[2];
-  b->sk = st[3];
-}
-
-// Called with autograd in force where the result is saved: the detached tensor then shares the version counter of the
-// caller's, and a change of the bias between forward and backward is found.
+// Called below autograd.  A contiguous fp32 bias is used as it is: no view is made of it, so its version counter is the
+// caller's, and a change between forward and backward is found.
 bool canonical_bias(const at::Tensor& bias, const Call& c, c10::Device dev, Bias* out) {
   if (!bias.defined()) return true;
-  const int64_t dim = bias.dim();
-  if (bias.device() != dev || dim < 2 || dim > 4 || bias.size(dim - 2) != c.n || bias.size(dim - 1) != c.n) return false;
+  const int64_t dim = bias.dim(), n = c.n;
+  if (bias.device() != dev || dim < 2 || dim > 4 || bias.size(dim - 2) != n || bias.size(dim - 1) != n) return false;
   const int64_t lh = dim >= 3 ? bias.size(dim - 3) : 1, lb = dim == 4 ? bias.size(0) : 1;
   if ((lh != 1 && lh != c.heads) || (lb != 1 && lb != c.batch)) return false;
-  at::Tensor v = bias.detach();
-  if (v.scalar_type() != at::kFloat) v = v.to(at::kFloat);
-  if (!v.is_contiguous()) v = v.contiguous();
-  out->t = dim == 4 ? v : v.view({lb, lh, c.n, c.n});
-  bias_strides(out);
+  out->t = (bias.scalar_type() == at::kFloat ? bias : bias.to(at::kFloat)).contiguous();
+  out->sb = lb == 1 ? 0 : lh * n * n;
+  out->sh = lh == 1 ? 0 : n * n;
+  out->sq = n;
+  out->sk = 1;
   return true;
 }
 
@@ -276,7 +268,7 @@ struct BackwardPlan {
     return p;
   }
 
-  // packed: q is the packed tensor, k and v stay undefined, bias is the canonical bias; else bias is the caller's (a 16-bit or
+  // packed: q is the packed tensor, k and v stay undefined, bias is the one in fp32; else bias is the caller's (a 16-bit or
   // expanded bias is kept as it is, and converted again by the backward)
   struct Saved { at::Tensor q, k, v, out, state, bias; };
 
@@ -302,7 +294,8 @@ struct BackwardPlan {
       // Sums over a broadcast axis and pairs that the causal rule leaves out need zeros.  Otherwise the kernels store every
       // element once, and clearing the tensor first is one more pass over it (537 MB at (1,8,4096,64)).
       const bool summed = (bias.sb == 0 && c.batch > 1) || (bias.sh == 0 && c.heads > 1);
-      dbias = (summed || c.causal) ? at::zeros_like(bias.t) : at::empty_like(bias.t);
+      dbias = new_tensor(bias_sizes, go, at::kFloat);
+      if (summed || c.causal) dbias.zero_();
     }
     View t[8];
     if (packed) {
@@ -331,7 +324,6 @@ struct BackwardPlan {
       run_backward(t, strided, bias, dbias, state, c, dev);
     }
     if (bias_grad) {
-      dbias = dbias.view(bias_sizes);
       result.back() = dbias.scalar_type() == bias_dtype ? dbias : dbias.to(bias_dtype);
     }
     return result;
@@ -446,11 +438,11 @@ at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
   const bool record = train && at::GradMode::is_enabled() &&
                       (q.requires_grad() || k.requires_grad() || v.requires_grad() || (bias.defined() && bias.requires_grad()));
   Bias canon;
-  if (!canonical_bias(bias, c, q.device(), &canon)) return {};
   std::array<at::Tensor, 3> in{q, k, v};
   at::Tensor out, state;
   {
     at::AutoDispatchBelowADInplaceOrView below;
+    if (!canonical_bias(bias, c, q.device(), &canon)) return {};
     View t[3], o;
     const bool strided = pick_layouts(in, t);
     out = strided ? new_like_layout(in[0], t[0]) : new_tensor(q.sizes(), q, q.scalar_type());
@@ -477,10 +469,10 @@ at::Tensor attention_packed(const at::Tensor& qkv, const at::Tensor& bias, Call 
     return {};
   const bool record = train && at::GradMode::is_enabled() && (qkv.requires_grad() || (bias.defined() && bias.requires_grad()));
   Bias canon;
-  if (!canonical_bias(bias, c, qkv.device(), &canon)) return {};
   at::Tensor out, state;
   {
     at::AutoDispatchBelowADInplaceOrView below;
+    if (!canonical_bias(bias, c, qkv.device(), &canon)) return {};
     out = new_bnhd(qkv, c.batch, c.heads, c.n, c.d);
     View in[3], o;
     packed_views(data_of(qkv), c, qkv.element_size(), in);
