@@ -297,7 +297,7 @@ extern "C" int elsa_debug_wait_timeout(uint64_t limit_ns, void* stream) {
 
 extern "C" int64_t elsa_kernel_launches(void) { return static_cast<int64_t>(g_kernel_launches.load()); }
 
-static bool tc_backward_ok(int dtype, int head_dim, int n_ctx, int bh, bool has_bias, unsigned flags);
+static bool tc_backward_ok(int dtype, int head_dim, int n_ctx, unsigned flags);
 static bool tc3_backward_ok(int dtype, int head_dim, int n_ctx, int bh, bool has_bias, unsigned flags);
 static bool tcw_backward_ok(int dtype, int head_dim, int n_ctx, int bh, bool has_bias, unsigned flags);
 
@@ -308,7 +308,7 @@ extern "C" int elsa_uses_tensor_cores_for(int dtype, int head_dim, int n_ctx, in
   if (n_ctx >= 1 && n_ctx <= 64 && win_tc_supported(dtype, head_dim, n_ctx, is_causal != 0)) return 1;
   const int bh = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(batch) * heads, 1 << 30));
   if (backward)
-    return (tc_backward_ok(dtype, head_dim, n_ctx, bh, has_bias != 0, 0u) || tc3_backward_ok(dtype, head_dim, n_ctx, bh, has_bias != 0, 0u) ||
+    return (tc_backward_ok(dtype, head_dim, n_ctx, 0u) || tc3_backward_ok(dtype, head_dim, n_ctx, bh, has_bias != 0, 0u) ||
             tcw_backward_ok(dtype, head_dim, n_ctx, bh, has_bias != 0, 0u)) ? 1 : 0;
   return (tc_forward_ok(dtype, head_dim, n_ctx, bh, has_bias != 0, 0u) || tc3_forward_ok(dtype, head_dim, n_ctx, bh, has_bias != 0, 0u) ||
           tcw_forward_ok(dtype, head_dim, n_ctx, bh, has_bias != 0, 0u)) ? 1 : 0;
@@ -555,12 +555,11 @@ extern "C" int elsa_twopass_forward_strided(const void* q, const void* k, const 
 }
 
 // ---- backward -------------------------------------------------------------------------------
-static bool tc_backward_ok(int dtype, int head_dim, int n_ctx, int bh, bool has_bias, unsigned flags) {
+static bool tc_backward_ok(int dtype, int head_dim, int n_ctx, unsigned flags) {
   if (flags & ELSA_FLAG_FORCE_SIMT) return false;
   // (the 16-bit backward has no rounding points to keep in step with a forward plan, and from 65 tokens on it is faster
   // than the FP32-FMA kernels at every batch size: 0.048 against 0.095 ms at (1,8,197,64))
-  (void)bh;
-  return n_ctx > 64 && bwd_tc_supported(dtype, head_dim, has_bias);
+  return n_ctx > 64 && bwd_tc_supported(dtype, head_dim);
 }
 
 // fp32 on the tensor cores (16-bit planes per operand): head dim up to 64, with or without a bias (and its gradient)
@@ -584,12 +583,12 @@ extern "C" int64_t elsa_backward_workspace_bytes(int dtype, int batch, int heads
                                                  int has_bias, int is_causal, unsigned flags) {
   (void)is_causal;
   if (!dtype_ok(dtype) || batch < 1 || heads < 1 || n_ctx < 0 || head_dim < 1 || head_dim > 128) return -1;
-  if (tc_backward_ok(dtype, head_dim, n_ctx, batch * heads, has_bias != 0, flags)) {
+  if (tc_backward_ok(dtype, head_dim, n_ctx, flags)) {
     // (a biased problem runs there only when dbias is asked for, else on the wide-head kernels: room for either)
     const int64_t tc = bwd_tc_workspace_bytes(batch * heads, n_ctx);
     return has_bias ? std::max(tc, bwd_tcw_workspace_bytes(batch * heads, n_ctx)) : tc;
   }
-  // (the fp32 tensor-core route is not taken when dbias is asked for: the larger of the two needs covers both)
+  // (a bias gradient asked for without a bias stays on the FP32-FMA kernels: the larger of the two needs covers both)
   if (tc3_backward_ok(dtype, head_dim, n_ctx, batch * heads, has_bias != 0, flags))
     return std::max(bwd_tc3_workspace_bytes(batch * heads, n_ctx, n_ctx), 2 * bwd_state_bytes(batch, heads, n_ctx));
   if (tcw_backward_ok(dtype, head_dim, n_ctx, batch * heads, has_bias != 0, flags))
@@ -621,7 +620,7 @@ static int backward_impl(const void* q, const void* k, const void* v, const void
   // d <= 64, 16-bit: the five-contraction kernel, for a biased problem only when its gradient is asked for.  It reads the bias
   // and writes dbias once, where the kernel of bwd_tcw.cu reads the bias twice, but adds dQ in arrival order; without a
   // bias gradient, or on request, the biased backward keeps the order-independent kernel (its dq repeats bit for bit).
-  const bool use_tc = (bias == nullptr) == (dbias == nullptr) && !(bias && (flags & ELSA_FLAG_REPEATABLE)) && tc_backward_ok(dtype, head_dim, n_ctx, batch * heads, bias != nullptr, flags);
+  const bool use_tc = (bias == nullptr) == (dbias == nullptr) && !(bias && (flags & ELSA_FLAG_REPEATABLE)) && tc_backward_ok(dtype, head_dim, n_ctx, flags);
   const bool use_tc3 = (dbias == nullptr || bias != nullptr) && tc3_backward_ok(dtype, head_dim, n_ctx, batch * heads, bias != nullptr, flags);
   // (the wide-head kernels also take biased problems, with or without a bias gradient)
   const bool use_tcw = !use_tc && !use_tc3 && (dbias == nullptr || bias != nullptr) &&
@@ -734,7 +733,7 @@ extern "C" int elsa_twopass_backward_shard(const void* q, const void* k_shard, c
   float* row_d = reinterpret_cast<float*>(ws);
   float* row_lse = reinterpret_cast<float*>(ws + bwd_state_bytes(batch, heads, n_ctx));
   // (the tensor-core kernels address the fp32 dQ of a shard as 64-wide rows)
-  const bool use_tc = n_keys > 0 && head_dim == 64 && tc_backward_ok(dtype, head_dim, n_ctx, batch * heads, false, flags);
+  const bool use_tc = n_keys > 0 && head_dim == 64 && tc_backward_ok(dtype, head_dim, n_ctx, flags);
   const bool use_tc3 = n_keys > 0 && n_keys <= n_ctx && tc3_backward_ok(dtype, head_dim, n_ctx, batch * heads, false, flags);
   const bool use_tcw = n_keys > 0 && tcw_backward_ok(dtype, head_dim, n_ctx, batch * heads, false, flags);
   int rc = ELSA_OK;

@@ -594,10 +594,7 @@ dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq, int n_ctx, 
 
 }  // namespace
 
-bool bwd_tc_supported(int dtype, int head_dim, bool has_bias) {
-  (void)has_bias;
-  return fold_tc_supported(dtype, head_dim, false);
-}
+bool bwd_tc_supported(int dtype, int head_dim) { return fold_tc_supported(dtype, head_dim, false); }
 
 int64_t bwd_tc_workspace_bytes(int bh, int n_ctx) {
   const int64_t n_pad = align_up(n_ctx, 128);
@@ -661,7 +658,7 @@ static int bwd_tc_t(const BwdParams& p, const void* out, Strides os, const float
 
 int bwd_tc(const BwdParams& p, const void* out, Strides os, const float* row_m, const float* row_z, void* workspace,
            int dtype, cudaStream_t st) {
-  if (!bwd_tc_supported(dtype, p.head_dim, p.bias != nullptr) || (p.dbias && !p.bias)) return ELSA_ERR_UNSUPPORTED;
+  if (!bwd_tc_supported(dtype, p.head_dim) || (p.dbias && !p.bias)) return ELSA_ERR_UNSUPPORTED;
   if (p.dq_f32 && p.head_dim != 64) return ELSA_ERR_UNSUPPORTED;   // the caller's fp32 dQ is the accumulator: 64-wide rows
   if (dtype == ELSA_F16) return bwd_tc_t<__half>(p, out, os, row_m, row_z, workspace, dtype, st);
   return bwd_tc_t<__nv_bfloat16>(p, out, os, row_m, row_z, workspace, dtype, st);

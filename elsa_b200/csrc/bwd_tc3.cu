@@ -8,14 +8,14 @@
 // accumulated over tiles in TMEM: every (query tile, key tile) pair gets fresh accumulators, and the running sums live
 // in the registers of the threads that drain them (ordinary round-to-nearest additions).  A resident dK / dV with a
 // streamed dQ (one kernel, five contractions) would need global atomics for dQ and more TMEM than there is, so the
-// work is done by two kernels of the same shape as the forward one, seven contractions per pair in all:
+// work is done by two bodies of the same shape as the forward kernel, in one launch, seven contractions per pair in all:
 //
 //   bwd3_dq_body      one CTA per 128-row QUERY tile, 128-key tiles streamed:
 //                       S  = Q K^T, dP = dO V^T       A = Q / dO planes (shared memory), B = K / V planes
 //                       dS = P (dP - D), P = 2^(S c - LSE)          four threads per query row
 //                       dQ_j = dS K                    A = dS planes (TMEM), B = the same K planes, MN-major
 //                     dQ = scale * sum_j dQ_j in registers, written once: no atomics, deterministic
-//   bwd3_dkv_body    one CTA per 128-row KEY tile, 64-query tiles streamed:
+//   bwd3_dkv_body     one CTA per 128-row KEY tile, 64-query tiles streamed:
 //                       S^T = K Q^T, dP^T = V dO^T     A = K / V planes (shared memory), B = Q / dO planes
 //                       P^T, dS^T                      four threads per key row; -LSE, -D of the tile's queries
 //                                                      arrive with the tile (bulk copies into a small ring)
@@ -65,7 +65,7 @@ struct Bwd3Params {
   int head_dim;                                 // real columns of the gradients (<= 64; the planes are zero-padded to 64)
   float scale, scale_log2;
   const float* bias; int64_t bsb, bsh, bsq, bsk;      // additive bias [.., N, N] (natural-log units) or null
-  float* dbias; int64_t dsb, dsh, dsq, dsk;           // its gradient (same addressing; zeroed by the caller) or null
+  float* dbias; int64_t dsb, dsh, dsq, dsk;           // its gradient (same addressing) or null
   int dbias_atomic;                                   // a broadcast axis: contributions are added atomically
   int* status;                                  // the device's status word (mapped host memory)
 };
@@ -377,8 +377,8 @@ __device__ __forceinline__ void bwd3_dq_body(const CUtensorMap& tmap_q, const CU
             if (kb + i > lim) ds[i] = 0.f;
         }
         if constexpr (BIAS) {
-          // dbias = dS (every (query, key) pair is visited exactly once by this kernel); pairs that the causal rule or
-          // the sequence length excludes hold zeros here, as the caller zeroed them
+          // dbias = dS: every (query, key) pair is stored exactly once, so only a summed axis (added atomically) and the
+          // causal rule (whole tiles above the diagonal are not visited) want a tensor that the caller cleared
           if (dbias_row && qi < N) {
             float* dp = dbias_row + static_cast<int64_t>(kb + koff) * prm.dsk;
             if (!prm.dbias_atomic && prm.dsk == 1 && kb + 32 <= NK && (reinterpret_cast<uintptr_t>(dp) & 31u) == 0) {

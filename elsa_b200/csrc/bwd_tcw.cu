@@ -1,7 +1,8 @@
 // Backward on the 5th-generation tensor cores for fp16 / bf16 inputs with a WIDE head, 64 < d <= 128 (multiples of 8),
 // causal or not, and for BIASED problems of any head dim up to 128 (bias and dbias are read / written in global memory
-// by the fold warps of the dQ kernel; with d <= 64 only the first half below exists): exact recompute from the saved
-// row statistics.  The head dim is handled as two 64-column
+// by the fold warps of the dQ body; with d <= 64 only the first half below exists): exact recompute from the saved
+// row statistics.  With d <= 64 and a bias gradient it is the slower but order-independent one (ELSA_FLAG_REPEATABLE); by
+// default such a problem runs on bwd_tc.cu.  The head dim is handled as two 64-column
 // halves of the same tensors (the second half zero-padded by the TMA box when d < 128).
 //
 // The kernel for d <= 64 (bwd_tc.cu) keeps S^T, dP^T, dV, dK and dQ of one key tile in TMEM; with 128 gradient columns
@@ -12,7 +13,7 @@
 //                       S  = Q_lo K_lo^T + Q_hi K_hi^T,  dP = dO_lo V_lo^T + dO_hi V_hi^T        (N = 128)
 //                       dS = P (dP - D), P = 2^(S c - LSE), rounded to the input type, into TMEM
 //                       dQ_h += dS K_h, h = lo, hi       accumulated in TMEM over the key tiles  (N = 64 each)
-//   bwdw_dkv_body    one CTA per 128-row KEY tile, 64-query tiles streamed:
+//   bwdw_dkv_body     one CTA per 128-row KEY tile, 64-query tiles streamed:
 //                       S^T = K_lo Q_lo^T + K_hi Q_hi^T, dP^T = V_lo dO_lo^T + V_hi dO_hi^T      (N = 64)
 //                       P^T, dS^T rounded to the input type, into TMEM
 //                       dV_h += P^T dO_h, dK_h += dS^T Q_h   accumulated in TMEM over the query tiles
@@ -61,7 +62,7 @@ struct BwdWParams {
   int n_halves;                                 // 1 when head_dim <= 64 (biased problems), else 2
   float scale, scale_log2;
   const float* bias; int64_t bsb, bsh, bsq, bsk;      // additive bias [.., N, N] (natural-log units) or null
-  float* dbias; int64_t dsb, dsh, dsq, dsk;           // its gradient (same addressing; zeroed by the caller) or null
+  float* dbias; int64_t dsb, dsh, dsq, dsk;           // its gradient (same addressing) or null
   int dbias_atomic;                                   // a broadcast axis: contributions are added atomically
   int* status;                                  // the device's status word (mapped host memory)
 };
@@ -303,8 +304,8 @@ __device__ __forceinline__ void bwdw_dq_body(const CUtensorMap& tmap_q, const CU
 #pragma unroll
         for (int i = 0; i < 32; i += 2) pk[i >> 1] = pack2<T>(dsv[i], dsv[i + 1]);
         if constexpr (BIAS) {
-          // dbias = dS (every (query, key) pair is visited exactly once by this kernel); pairs that the causal rule or
-          // the sequence length excludes hold zeros here, as the caller zeroed them
+          // dbias = dS: every (query, key) pair is stored exactly once, so only a summed axis (added atomically) and the
+          // causal rule (whole tiles above the diagonal are not visited) want a tensor that the caller cleared
           if (dbias_row && qi < N) {
             float* dp = dbias_row + static_cast<int64_t>(kb + koff) * prm.dsk;
             if (!prm.dbias_atomic && prm.dsk == 1 && kb + 32 <= NK && (reinterpret_cast<uintptr_t>(dp) & 31u) == 0) {

@@ -99,7 +99,7 @@ int fold_tc3_split_many(int n, const void* const* x, const Strides* st, void* co
                         int heads, int cols, cudaStream_t stream, const SplitStats* stats = nullptr);
 int fold_tc3(const FoldParams& p, cudaStream_t st);
 // tcgen05 backward (bwd_tc.cu); workspace = padded D / LSE vectors + fp32 dQ accumulator
-bool bwd_tc_supported(int dtype, int head_dim, bool has_bias);
+bool bwd_tc_supported(int dtype, int head_dim);   // with or without a bias
 int64_t bwd_tc_workspace_bytes(int bh, int n_ctx);
 int bwd_tc(const BwdParams& p, const void* out, Strides os, const float* row_m, const float* row_z, void* workspace,
            int dtype, cudaStream_t st);
