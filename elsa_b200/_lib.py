@@ -99,10 +99,11 @@ def _load_host():
     except ImportError as exc:
         why = f"does not load ({exc})"
     else:
-        if mod.torch_version == torch.__version__:
+        built_for = getattr(mod, "torch_version", "an unknown version")     # (a file of an earlier build says nothing)
+        if built_for == torch.__version__:
             mod.bind({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in _HOST_ENTRIES})
             return mod
-        why = f"was built for torch {mod.torch_version}, this is {torch.__version__}"
+        why = f"was built for torch {built_for}, this is {torch.__version__}"
     warnings.warn(f"elsa_b200/_host.so {why}: operators take their general path, with the same kernels and more host time per "
                   "call; build it with `python -m elsa_b200.build`", RuntimeWarning, stacklevel=4)
     return None

@@ -139,7 +139,7 @@ def test_host_path_is_rebuilt_for_another_torch(lib, monkeypatch, tmp_path):
     assert build.host_needs_build()
 
 
-@pytest.mark.parametrize("how", ["missing", "other torch", "built"])
+@pytest.mark.parametrize("how", ["missing", "other torch", "unmarked", "built"])
 def test_host_path_that_does_not_fit_is_left_out(lib, monkeypatch, how):
     import sys
     import warnings
@@ -153,6 +153,9 @@ def test_host_path_that_does_not_fit_is_left_out(lib, monkeypatch, how):
         monkeypatch.delattr(elsa_b200, "_host", raising=False)
     elif how == "other torch":
         monkeypatch.setattr(torch, "__version__", "0.0.1")
+    elif how == "unmarked":
+        from elsa_b200 import _host
+        monkeypatch.delattr(_host, "torch_version")
     with warnings.catch_warnings(record=True) as caught:
         warnings.simplefilter("always")
         first, second = _lib.host(), _lib.host()
