@@ -350,7 +350,7 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const float* bias_row = nullptr;
     if constexpr (BIAS) {
       const int bi = bh / prm.heads, hi = bh - bi * prm.heads;
-      bias_row = prm.bias + bi * prm.bsb + hi * prm.bsh + static_cast<int64_t>(min(qi, prm.n_ctx - 1)) * prm.bsq;
+      bias_row = prm.bias + bi * prm.bsb + hi * prm.bsh + static_cast<int64_t>(min(qi, prm.n_ctx - 1)) * prm.bsq + koff * prm.bsk;
     }
     float m_ref = -CUDART_INF_F, m_true = -CUDART_INF_F, zsum = 0.f;   // zsum: this thread's 32 columns only, times kPlaneUnit
     float o_run[16];                                        // running sum of O over the key tiles (columns 16 cq ...), relative to m_ref
@@ -375,10 +375,30 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (j + 1 < n_t) { ik_next = inv_k[j + 1]; iv_next = inv_v[j + 1]; }
       // with a bias the scores are moved to the log2 domain at once (s c + b log2 e) and the scale below becomes 1
       const float cc = BIAS ? 1.f : c;
-      if (!mbar_wait_warp(bar_s, j & 1, &abort_flag, prm.status, BAR_S)) { alive = false; break; }
-      tc_fence_after();
+      const int k0 = k_begin + j * 128 + 32 * cq;           // first (local) key of this thread's columns
       float sv[32];
-      {
+      if constexpr (BIAS) {
+        // the bias is asked for before the scores are waited for, and the scores are read 16 columns at a time: the 32 bias
+        // values and 32 scores at once do not fit the 96 registers of a thread (and with the scales of the key tiles the
+        // loads had come to wait for one another: fp32 (1,8,2047,64) with a per-head bias 255 us, now 76; on 32-byte rows,
+        // N = 4096, 253 and 202)
+        float b0[16], b1[16];
+        load_bias16(b0, bias_row, prm.bsk, k0, k_end);
+        load_bias16(b1, bias_row, prm.bsk, k0 + 16, k_end);
+        if (!mbar_wait_warp(bar_s, j & 1, &abort_flag, prm.status, BAR_S)) { alive = false; break; }
+        tc_fence_after();
+        uint32_t r[16];
+        tmem_ld16(tS + lane_off + 32 * cq, r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sv[i] = fmaf(__uint_as_float(r[i]), c, b0[i] * 1.4426950408889634f);
+        tmem_ld16(tS + lane_off + 32 * cq + 16, r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sv[16 + i] = fmaf(__uint_as_float(r[i]), c, b1[i] * 1.4426950408889634f);
+      } else {
+        if (!mbar_wait_warp(bar_s, j & 1, &abort_flag, prm.status, BAR_S)) { alive = false; break; }
+        tc_fence_after();
         uint32_t r[32];
         tmem_ld32(tS + lane_off + 32 * cq, r);
         tmem_wait_ld();
@@ -387,26 +407,6 @@ fold_tc3_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       tc_fence_before();
       mbar_arrive_warp(bar_sfree, lane);        // S may be overwritten with the next tile's scores
-      const int k0 = k_begin + j * 128 + 32 * cq;           // first (local) key of this thread's columns
-      if constexpr (BIAS) {
-        const float* bp = bias_row + static_cast<int64_t>(k0 + koff) * prm.bsk;
-        if (prm.bsk == 1 && k0 + 32 <= k_end && (reinterpret_cast<uintptr_t>(bp) & 31u) == 0) {
-          // the thread's 128 bytes of the bias row as four whole sectors (a warp's 32 rows are 32 different lines)
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            float b8[8];
-            ld_global_v8(bp + 8 * g, b8);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sv[8 * g + e] = fmaf(sv[8 * g + e], c, b8[e] * 1.4426950408889634f);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float b = (k0 + i < k_end) ? bp[i * prm.bsk] : 0.f;
-            sv[i] = fmaf(sv[i], c, b * 1.4426950408889634f);
-          }
-        }
-      }
       const bool tail = k_begin + j * 128 + 128 > k_end;
       const bool diag = prm.is_causal && (k_begin + j * 128 + koff + 127 > q0);
       if (tail || diag) {

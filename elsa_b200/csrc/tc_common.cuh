@@ -313,6 +313,29 @@ __device__ __forceinline__ void st_global_v8(float* p, const float (&r)[8]) {
                ::"l"(p), "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]) : "memory");
 }
 
+// 16 consecutive keys of one bias row: row + stride * k ...  Every load is unconditional (a key at or beyond k_end reads the
+// last one; its score is masked later): with a condition each element is a basic block and a load's latency of its own.
+__device__ __forceinline__ void load_bias16(float (&b)[16], const float* row, int64_t stride, int k, int k_end) {
+  if (stride == 1 && k + 16 <= k_end) {
+    const float* p = row + k;
+    if ((reinterpret_cast<uintptr_t>(p) & 31u) == 0) {
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        float b8[8];
+        ld_global_v8(p + 8 * g, b8);          // whole 32-byte sectors (a warp's 32 rows are 32 different lines)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) b[8 * g + e] = b8[e];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) b[i] = __ldg(p + i);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) b[i] = __ldg(row + stride * min(k + i, k_end - 1));
+  }
+}
+
 // ---- fp32 operands as a few 16-bit planes -----------------------------------------------------------------------
 // ELSA_FP32_PLANES == 3: x = a0 + a1 + a2 with three bf16 terms (8 + 8 + 8 significant bits, the full exponent range;
 //   six cross products of weight >= 2^-16 per contraction).

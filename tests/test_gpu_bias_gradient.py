@@ -76,3 +76,29 @@ def test_rows_without_a_key_get_zero_gradients(n, d, dtype, shared):
     for g, w in zip(got, want):
         assert torch.isfinite(g).all()
         assert (g.double() - w).norm() <= LIMIT[dtype] * w.norm()
+
+
+@pytest.mark.parametrize("n,part_width", [(512, 0), (516, 128), (520, 0), (527, 256), (639, 128), (1025, 384)])
+@pytest.mark.parametrize("form", ["rows", "offset", "transposed"])
+@pytest.mark.parametrize("causal", [False, True])
+def test_fp32_tensor_core_fold_reads_a_bias_of_any_alignment(n, part_width, form, causal):
+    """16 keys at a time: whole sectors on 32-byte boundaries, single loads off them, clamped ones at a partition's end and for a
+    bias whose keys are not contiguous (C ABI only)."""
+    lib = _lib.load()
+    b, h, d = 1, 2, 64
+    q, k, v, _, bias = _problem(b, h, n, d, torch.float32)
+    if form == "offset":
+        bias = torch.cat([bias.new_zeros(1), bias.reshape(-1)])[1:].view_as(bias)
+    elif form == "transposed":
+        bias = bias.mT.contiguous().mT
+    out, row_m, row_z = torch.full_like(q, float("nan")), q.new_empty(b * h, n), q.new_empty(b * h, n)
+    need = lib.elsa_forward_workspace_bytes(0, 0, b, h, n, d, 1, int(causal), part_width, 0, 0)
+    ws = torch.empty(max(need, 256), device="cuda", dtype=torch.uint8)
+    rc = lib.elsa_twopass_forward(q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(), *bias.stride(), out.data_ptr(), row_m.data_ptr(),
+                                  row_z.data_ptr(), ws.data_ptr(), ws.numel(), 0, 0, b, h, n, d, int(causal), part_width, 0, 0, _lib.raw_stream(q.device))
+    assert rc == 0
+    s = q.double() @ k.double().mT * d ** -0.5 + bias.double()
+    if causal:
+        s = s.masked_fill(torch.ones(n, n, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    want = torch.softmax(s, -1) @ v.double()
+    assert (out.double() - want).norm() <= 1e-6 * want.norm()      # the bound of the unbiased fold
