@@ -313,7 +313,7 @@ __device__ __forceinline__ void bwd3_dq_body(const CUtensorMap& tmap_q, const CU
     if constexpr (BIAS) {
       const int bi = bh / prm.heads, hi = bh - bi * prm.heads;
       const int qrow = min(qi, N - 1);         // rows beyond N are never stored: any valid address will do
-      bias_row = prm.bias + bi * prm.bsb + hi * prm.bsh + static_cast<int64_t>(qrow) * prm.bsq;
+      bias_row = prm.bias + bi * prm.bsb + hi * prm.bsh + static_cast<int64_t>(qrow) * prm.bsq + koff * prm.bsk;
       if (prm.dbias) dbias_row = prm.dbias + bi * prm.dsb + hi * prm.dsh + static_cast<int64_t>(qrow) * prm.dsq;
     }
     float dq_run[16];
@@ -331,45 +331,44 @@ __device__ __forceinline__ void bwd3_dq_body(const CUtensorMap& tmap_q, const CU
     for (int j = 0; alive && j < n_t; ++j) {
       const float ik = ik_next, c = c_q * ik, idp = i_do * iv_next;
       if (j + 1 < n_t) { ik_next = inv_k[j + 1]; iv_next = inv_v[j + 1]; }
+      const int kb = j * 128 + 32 * cq;                     // first (local) key of this thread's columns
+      float ds[32];
+      // dS of 16 columns at a time with a bias (it, S, dP and dS of 32 do not fit the 96 registers of a thread: 600 bytes of
+      // spill stores, now 252), else of 32; the bias of the first 16 is asked for before the wait, that of the second 16
+      // before the first are worked on.  fp32 (1,8,4096,64) with a per-head bias and its gradient 1084 -> 903 us, 2047 keys
+      // (rows off 32-byte boundaries, conditional loads and stores before) 604 -> 427
+      constexpr int kCols = BIAS ? 16 : 32;
+      float bb[16];
+      if constexpr (BIAS) load_bias16(bb, bias_row, prm.bsk, kb, NK);
       if (!mbar_wait_warp(bar_sdp, j & 1, &abort_flag, prm.status, BAR_SDP)) { alive = false; break; }
       tc_fence_after();
-      float ds[32];
       {
-        uint32_t rs[32], rp[32];
-        tmem_ld32(tS + lane_off + 32 * cq, rs);
-        tmem_ld32(tdP + lane_off + 32 * cq, rp);
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive_warp(bar_sfree, lane);      // S and dP may be overwritten with the next tile's
-        const int kb = j * 128 + 32 * cq;                   // first (local) key of this thread's columns
         const bool masked = (j * 128 + 128 > NK) || (prm.is_causal && (j * 128 + koff + 127 > q0));
         const int lim = prm.is_causal ? min(NK - 1, qi - koff) : NK - 1;   // last admissible (local) key of this row
-        float ab[32];                                       // bias log2(e) - LSE of this thread's 32 keys
 #pragma unroll
-        for (int i = 0; i < 32; ++i) ab[i] = nlse;
-        if constexpr (BIAS) {
-          const float* bp = bias_row + static_cast<int64_t>(kb + koff) * prm.bsk;
-          if (prm.bsk == 1 && kb + 32 <= NK && (reinterpret_cast<uintptr_t>(bp) & 31u) == 0) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              float b8[8];
-              ld_global_v8(bp + 8 * g, b8);      // whole 32-byte sectors (a warp's 32 rows are 32 different lines)
-#pragma unroll
-              for (int e = 0; e < 8; ++e) ab[8 * g + e] = fmaf(b8[e], 1.4426950408889634f, nlse);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (kb + i < NK) ab[i] = fmaf(bp[i * prm.bsk], 1.4426950408889634f, nlse);
+        for (int h = 0; h < 32; h += kCols) {
+          uint32_t rs[kCols], rp[kCols];
+          if constexpr (BIAS) { tmem_ld16(tS + lane_off + 32 * cq + h, rs); tmem_ld16(tdP + lane_off + 32 * cq + h, rp); }
+          else { tmem_ld32(tS + lane_off + 32 * cq, rs); tmem_ld32(tdP + lane_off + 32 * cq, rp); }
+          tmem_wait_ld();
+          if (h + kCols == 32) {
+            tc_fence_before();
+            mbar_arrive_warp(bar_sfree, lane);  // S and dP may be overwritten with the next tile's
           }
-        }
-        // (packed pairs and a mask loop of its own: the fold warps issue in 50 to 64 % of the cycles, their instructions count)
+          float ab[kCols];                      // bias log2(e) - LSE
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float2 x = __ffma2_rn(pair_of(rs, i), make_float2(c, c), make_float2(ab[i], ab[i + 1]));
-          const float2 t = __ffma2_rn(pair_of(rp, i), make_float2(idp, idp), make_float2(nd, nd));
-          const float2 d2 = __fmul2_rn(make_float2(fast_exp2(x.x), fast_exp2(x.y)), t);
-          ds[i] = d2.x; ds[i + 1] = d2.y;
+          for (int i = 0; i < kCols; ++i) ab[i] = BIAS ? fmaf(bb[i & 15], 1.4426950408889634f, nlse) : nlse;
+          if constexpr (BIAS) {
+            if (h == 0) load_bias16(bb, bias_row, prm.bsk, kb + 16, NK);
+          }
+          // (packed pairs and a mask loop of its own: the fold warps issue in half of the cycles, their instructions count)
+#pragma unroll
+          for (int i = 0; i < kCols; i += 2) {
+            const float2 x = __ffma2_rn(pair_of(rs, i), make_float2(c, c), make_float2(ab[i], ab[i + 1]));
+            const float2 t = __ffma2_rn(pair_of(rp, i), make_float2(idp, idp), make_float2(nd, nd));
+            const float2 d2 = __fmul2_rn(make_float2(fast_exp2(x.x), fast_exp2(x.y)), t);
+            ds[h + i] = d2.x; ds[h + i + 1] = d2.y;
+          }
         }
         if (masked) {
 #pragma unroll
@@ -381,13 +380,18 @@ __device__ __forceinline__ void bwd3_dq_body(const CUtensorMap& tmap_q, const CU
           // causal rule (whole tiles above the diagonal are not visited) want a tensor that the caller cleared
           if (dbias_row && qi < N) {
             float* dp = dbias_row + static_cast<int64_t>(kb + koff) * prm.dsk;
-            if (!prm.dbias_atomic && prm.dsk == 1 && kb + 32 <= NK && (reinterpret_cast<uintptr_t>(dp) & 31u) == 0) {
+            if (!prm.dbias_atomic && prm.dsk == 1 && kb + 32 <= NK) {
+              if ((reinterpret_cast<uintptr_t>(dp) & 31u) == 0) {
 #pragma unroll
-              for (int g = 0; g < 4; ++g) {
-                float d8[8];
+                for (int g = 0; g < 4; ++g) {
+                  float d8[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) d8[e] = ds[8 * g + e];
-                st_global_v8(dp + 8 * g, d8);
+                  for (int e = 0; e < 8; ++e) d8[e] = ds[8 * g + e];
+                  st_global_v8(dp + 8 * g, d8);
+                }
+              } else {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) dp[i] = ds[i];
               }
             } else {
 #pragma unroll

@@ -102,3 +102,30 @@ def test_fp32_tensor_core_fold_reads_a_bias_of_any_alignment(n, part_width, form
         s = s.masked_fill(torch.ones(n, n, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
     want = torch.softmax(s, -1) @ v.double()
     assert (out.double() - want).norm() <= 1e-6 * want.norm()      # the bound of the unbiased fold
+
+
+@pytest.mark.parametrize("n,d", [(516, 64), (640, 64), (1025, 40), (130, 64)])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("form", ["rows", "offset", "transposed"])
+def test_a_dense_gradient_of_any_alignment(n, d, dtype, form):
+    """As `test_a_dense_gradient_is_stored_entry_by_entry`, with bias and gradient off 16-byte boundaries or key by key."""
+    lib = _lib.load()
+    b, h = 1, 2
+    q, k, v, do, bias = _problem(b, h, n, d, dtype)
+    out, row_m, row_z = E.twopass_attention_with_state(q, k, v, bias=bias)
+
+    def laid_out(t):
+        if form == "offset":
+            return torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view_as(t)
+        return t.mT.contiguous().mT if form == "transposed" else t
+
+    used, dbias = laid_out(bias), laid_out(torch.full_like(bias, float("nan")))
+    dq, dk, dv = (torch.full_like(q, float("nan")) for _ in range(3))
+    dt = _lib.dtype_code(dtype)
+    ws = torch.empty(max(lib.elsa_backward_workspace_bytes(dt, b, h, n, d, 1, 0, 0), 256), device="cuda", dtype=torch.uint8)
+    rc = lib.elsa_twopass_backward(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), do.data_ptr(), row_m.data_ptr(), row_z.data_ptr(),
+                                   used.data_ptr(), *used.stride(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), dbias.data_ptr(), *dbias.stride(),
+                                   ws.data_ptr(), ws.numel(), dt, b, h, n, d, 0, 0, _lib.raw_stream(q.device))
+    assert rc == 0
+    for g, w in zip((dq, dk, dv, dbias), _fp64(q, k, v, bias, do)):
+        assert (g.double() - w).norm() <= LIMIT[dtype] * w.norm()
