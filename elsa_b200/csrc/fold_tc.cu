@@ -25,9 +25,10 @@
 // max is tracked separately and the summary is renormalised to it in the epilogue, so the stored
 // (m, z, s) is the same monoid element the FP32-FMA kernel produces.
 //
-// Two changes took (1,8,16384,64) fp16 from 0.700 to 0.659 ms, causal bf16 from 0.407 to 0.383, (8,3,4097,64) from 0.173
-// to 0.157 and (64,3,197,64) from 20.5 to 18.6 us: the issuing warps run warp-uniform code (elect_one in tc_common.cuh),
-// and tile 1 starts half a period after tile 0.  Cycles per key tile and row: exponentials and P stores 1290 (1165 with
+// Four changes, measured together, took (1,8,16384,64) fp16 from 0.700 to 0.659 ms, causal bf16 from 0.407 to 0.383,
+// (8,3,4097,64) from 0.173 to 0.157 and (64,3,197,64) from 20.5 to 18.6 us: the issuing warps run warp-uniform code (elect_one
+// in tc_common.cuh; alone 0.700 -> 0.665), tile 1 starts half a period after tile 0, the scores are read in two halves (the
+// maximum of the first while the second is on its way), and barriers count warps instead of threads.  Cycles per key tile and row: exponentials and P stores 1290 (1165 with
 // the ex2 unit to itself), waits, TMEM loads and the maximum 1030; the period of a tile is 2565, so the ex2 unit is at
 // 80 %.  Every n-th pair of exponentials on the FMA pipe (n = 4, 8, 16) gains nothing at this point.
 //
