@@ -283,7 +283,7 @@ struct BackwardPlan {
     check_unpacked(s.state, {2 * padded_rows(c)}, at::kFloat, dev);
     const at::Tensor state = aligned(s.state);
     Bias bias;
-    if (s.bias.defined()) {
+    if (!saved_bias_sizes.empty()) {
       check_unpacked(s.bias, saved_bias_sizes, saved_bias_dtype, dev);
       canonical_bias(s.bias, c, dev, &bias);
     }
